@@ -165,9 +165,10 @@ class Plan:
     ``info["nf1"]``, ``info["nf2"]`` give the lengths in use. ``transpose`` is "tma" (the NUFFT's
     fine-row transposes load their tiles with TMA tensor copies where the layout allows, the
     default) or "plain" (plain loads only; the results are the same bit for bit). ``spread`` is
-    "registers" (the spreading holds each bin's whole tile in registers where it fits, the
-    default) or "window" (a sliding window of the kernel's rows); both add the same values in
-    the same order.
+    "registers" (the default) or "window" (a sliding window of the kernel's rows). By default
+    FP64 plans spread on the matrix instruction; FP32 grids and ``deterministic=True`` hold each
+    bin's whole tile in registers where it fits and add the same values in the same order as
+    the window.
     ``deterministic=True`` makes adjoints bitwise reproducible run to run (fixed-order sums in
     the ring pass and the spreading) at some cost in speed; by default floating-point atomic
     additions let two adjoints differ at round-off.

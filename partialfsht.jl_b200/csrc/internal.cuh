@@ -303,6 +303,11 @@ struct NufftGrid {
     int gap_lo = 0, gap_hi = 0, gap_ok = 0;
     int plain_transpose = 0;   // 1: the plain-load transposes only
     int spread_reg = 1;        // spreading holds each bin's tile in registers where it fits
+    // spreading (mma) and interpolation (mma_interp) on the matrix instruction (nufft_mma.cu): the
+    // points by blocks of blk_cols origin columns, strips of 4 origin rows, columns, in groups
+    // of 8 slots; nitems work items of at most item_rows origin rows
+    int mma = 0, mma_interp = 0;
+    int blk_cols = 1, item_rows = 1 << 20, nitems = 0;
     int interp_pipe = 1;       // one-transform interpolation copies the next group's tile ahead
 };
 
@@ -315,6 +320,9 @@ struct NufftDev {
     DevBuf sorder;    // int32 nbusy: non-empty bins by spreading colour, most points first in each
     DevBuf bslot;     // int4 nbusy: (bin, first point, end, 0) in binorder's order
     DevBuf sslot;     // int4 nbusy: the same in sorder's order
+    DevBuf items;     // int4 nitems: first origin row and column, slot range (g.mma)
+    DevBuf soff;      // double2: the slots' point offsets from their windows' first cells
+    DevBuf smeta;     // int2: the slots' words (nufft_mma.cu) and original indices (-1: empty slot)
     DevBuf ipts;      // double2: pts in the interpolation's order (each group's points dealt over
     DevBuf iperm;     // int32    their shared-memory bank class), and their original indices
     DevBuf colp2;     // int32 ncols: fine column of each mode column
@@ -335,6 +343,21 @@ struct NufftDev {
 
 // bounded device-side waits that gave up (the TMA row transposes), on the current device
 int tma_timeouts(int* out);
+
+// FP64 interpolation and spreading on the matrix instruction (nufft_mma.cu): the columns of a
+// window for kernel width w, and the two passes
+int mma_tile_cols(int w);
+int mma_max_advance();
+struct MmaGroup {
+    int first, n;  // sorted points [first, first + n), n <= 8
+    int strip;     // strip of the first of them
+    int col;       // first origin column of the block
+    int advance;   // strips from the group before it in its item
+};
+int mma_fill_slots(const NufftGrid& g, NufftDev& d, const double2* gg, const int* sidx,
+                   const MmaGroup* groups, int64_t nslots, cudaStream_t s);
+int interp_mma(const NufftGrid& g, NufftDev& d, double2* f, int B, cudaStream_t s);
+int spread_mma(const NufftGrid& g, NufftDev& d, const double2* f, int B, cudaStream_t s);
 
 // transform points (x = stretched colatitude, y = longitude; both radians) into grid
 // coordinates, sort them into bins, fill pts/perm/binstart. x,y are device arrays.

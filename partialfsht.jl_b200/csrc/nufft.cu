@@ -25,8 +25,8 @@
 #include <mutex>
 #include <tuple>
 
-#include "es_horner_table.h"
 #include "internal.cuh"
+#include "nufft_dev.cuh"
 #include "tma.cuh"
 
 namespace pf {
@@ -159,12 +159,14 @@ int minmax_device(const double* x, int64_t M, double* mn, double* mx, cudaStream
 // Bins are aligned to the kernel's first cell (origin) i0 = ceil(g - w/2) of each point:
 // bin (br, bc) holds the points with origin row in [br BR, br BR + BR) and origin column in
 // [bc BC, bc BC + BC) (columns, and rows when every row is kept, taken modulo the grid).
-// Within a bin the points are sorted by origin row, then origin column.
+// Within a bin the points are sorted by origin row, then origin column. With `strips` (the order
+// of nufft_mma.cu, bins of 4 rows) the bins of one block of columns follow each other and the
+// points of a bin are sorted by origin column, then row.
 __global__ void bin_keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
                                 int64_t M, double s1, double s2, int row0, int row_wrap,
                                 int nf1, int nf2, int nrows, int w, int bin_rows, int bin_cols,
-                                int nbr, int nbc, double2* __restrict__ g, int* __restrict__ key,
-                                int* __restrict__ idx, int* __restrict__ counts) {
+                                int nbr, int nbc, int strips, double2* __restrict__ g,
+                                int* __restrict__ key, int* __restrict__ idx, int* __restrict__ counts) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M;
          i += (int64_t)gridDim.x * blockDim.x) {
         double g1 = x[i] * s1;
@@ -184,9 +186,10 @@ __global__ void bin_keys_kernel(const double* __restrict__ x, const double* __re
         c = ((c % nf2) + nf2) % nf2;
         const int br = min(r / bin_rows, nbr - 1);
         const int bc = min(c / bin_cols, nbc - 1);
-        const int k = br * nbc + bc;
+        const int k = strips ? bc * nbr + br : br * nbc + bc;
+        const int rr = r - br * bin_rows, cc = c - bc * bin_cols;
         g[i] = make_double2(g1, g2);
-        key[i] = (k * bin_rows + (r - br * bin_rows)) * bin_cols + (c - bc * bin_cols);
+        key[i] = strips ? (k * bin_cols + cc) * bin_rows + rr : (k * bin_rows + rr) * bin_cols + cc;
         idx[i] = (int)i;
         atomicAdd(counts + k, 1);
     }
@@ -202,64 +205,194 @@ __global__ void gather_points_kernel(const double2* __restrict__ g, const int* _
     }
 }
 
-// bin offsets on the host (nbins + 1)
-static std::vector<int> binstart_host(const NufftGrid& g, const NufftDev& d, cudaStream_t s) {
-    std::vector<int> bs((size_t)g.nbr * g.nbc + 1, 0);
-    if (cudaMemcpyAsync(bs.data(), d.binstart.p, sizeof(int) * bs.size(), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        bs.clear();
-    return bs;
-}
-
 // The interpolation's order of the points (ipts / iperm): within each interpolation group, the
 // points dealt round-robin over the shared-memory bank class of their tile origin (element
 // offset (r0 TC + c0) mod KM, KM elements per 128 bytes), so that the KM lanes that read the
 // tile together in one shared-memory phase start at different banks and each tap's loads need
-// no replay. The group's point range is unchanged.
-int interp_point_order(const NufftGrid& g, NufftDev& d, const std::vector<int>& bs, cudaStream_t s) {
-    const int64_t M = g.M;
-    if (bs.empty()) {
-        set_error("copying the NUFFT bin offsets failed");
-        return 4;
-    }
-    std::vector<double2> pts(M);
-    std::vector<int> perm(M);
-    PF_CUDA(cudaMemcpyAsync(pts.data(), d.pts.p, sizeof(double2) * M, cudaMemcpyDeviceToHost, s));
-    PF_CUDA(cudaMemcpyAsync(perm.data(), d.perm.p, sizeof(int) * M, cudaMemcpyDeviceToHost, s));
-    PF_CUDA(cudaStreamSynchronize(s));
-    const int W = g.w, KM = g.fp32 ? 16 : 8;
-    const int G = g.igroup, TS = (G * g.bin_cols + W - 1) | 1;  // the kernel's tile row stride
-    std::vector<double2> opts(M);
-    std::vector<int> operm(M);
-    std::vector<std::vector<int>> bucket(KM);
-#pragma omp parallel for schedule(dynamic, 16) num_threads(16) firstprivate(bucket) if (M > 100000)
-    for (int q = 0; q < g.nbr * g.nsbc; ++q) {
-        const int br = q / g.nsbc, sg = q % g.nsbc;
-        const int a = bs[br * g.nbc + sg * G], e = bs[br * g.nbc + std::min(g.nbc, sg * G + G)];
-        const int tr0 = br * g.bin_rows, tc0 = sg * G * g.bin_cols;
-        for (auto& v : bucket) v.clear();
-        for (int i = a; i < e; ++i) {
-            int r = (int)std::ceil(pts[i].x - 0.5 * W);
-            if (g.row_wrap) r = ((r % g.nrows) + g.nrows) % g.nrows;
-            int c = (int)std::ceil(pts[i].y - 0.5 * W);
-            c = ((c % g.nf2) + g.nf2) % g.nf2;
-            const int64_t off = (int64_t)(r - tr0) * TS + (c - tc0);
-            bucket[(int)(((off % KM) + KM) % KM)].push_back(i);
+// no replay. The group's point range is unchanged. A warp per group: the class sizes, then each
+// point's rank in its class, which give its place.
+constexpr int kDealWarps = 8;
+__global__ void __launch_bounds__(kDealWarps * 32)
+deal_points_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
+                   const int* __restrict__ binstart, int ngroups, int nbc, int nsbc, int G, int BR, int BC,
+                   int W, int KM, int nrows, int nf2, int row_wrap, double2* __restrict__ opts,
+                   int* __restrict__ operm) {
+    __shared__ int cnt_s[kDealWarps][16], run_s[kDealWarps][16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q = blockIdx.x * kDealWarps + warp;
+    if (q >= ngroups) return;
+    const int br = q / nsbc, sg = q % nsbc;
+    const int a = binstart[br * nbc + sg * G], e = binstart[br * nbc + min(nbc, sg * G + G)];
+    const int tr0 = br * BR, tc0 = sg * G * BC, TS = (G * BC + W - 1) | 1;  // the kernel's tile row stride
+    int *cnt = cnt_s[warp], *run = run_s[warp];
+    if (lane < 16) cnt[lane] = run[lane] = 0;
+    __syncwarp();
+    auto cls = [&](double2 p) {
+        int r = (int)ceil(p.x - 0.5 * W), c = (int)ceil(p.y - 0.5 * W);
+        if (row_wrap) r = wrap(r, nrows);
+        c = wrap(c, nf2);
+        const int o = ((r - tr0) * TS + (c - tc0)) % KM;
+        return o < 0 ? o + KM : o;
+    };
+    for (int i = a + lane; i < e; i += 32) atomicAdd(cnt + cls(pts[i]), 1);
+    __syncwarp();
+    for (int base = a; base < e; base += 32) {
+        const int i = base + lane;
+        const bool on = i < e;
+        const double2 p = on ? pts[i] : make_double2(0.0, 0.0);
+        const int k = on ? cls(p) : 16;
+        const unsigned same = __match_any_sync(0xffffffffu, k);
+        const int before = __popc(same & ((1u << lane) - 1));
+        if (on) {
+            const int rank = run[k] + before;
+            int o = a;
+            for (int j = 0; j < KM; ++j) o += min(cnt[j], rank) + (j < k && cnt[j] > rank ? 1 : 0);
+            opts[o] = p;
+            operm[o] = perm[i];
         }
-        int o = a;
-        for (size_t j = 0; o < e; ++j)
-            for (int k = 0; k < KM; ++k)
-                if (j < bucket[k].size()) {
-                    opts[o] = pts[bucket[k][j]];
-                    operm[o] = perm[bucket[k][j]];
-                    ++o;
-                }
+        __syncwarp();
+        if (on && before == 0) run[k] += __popc(same);
+        __syncwarp();
     }
-    PF_TRY(d.ipts.alloc(sizeof(double2) * std::max<int64_t>(M, 1)));
-    PF_TRY(d.iperm.alloc(sizeof(int) * std::max<int64_t>(M, 1)));
-    PF_CUDA(cudaMemcpyAsync(d.ipts.p, opts.data(), sizeof(double2) * M, cudaMemcpyHostToDevice, s));
-    PF_CUDA(cudaMemcpyAsync(d.iperm.p, operm.data(), sizeof(int) * M, cudaMemcpyHostToDevice, s));
+}
+
+static int interp_point_order(const NufftGrid& g, NufftDev& d, const double2* pts, const int* perm, cudaStream_t s) {
+    PF_TRY(d.ipts.alloc(sizeof(double2) * std::max<int64_t>(g.M, 1)));
+    PF_TRY(d.iperm.alloc(sizeof(int) * std::max<int64_t>(g.M, 1)));
+    const int ngroups = g.nbr * g.nsbc;
+    deal_points_kernel<<<(ngroups + kDealWarps - 1) / kDealWarps, kDealWarps * 32, 0, s>>>(
+        pts, perm, d.binstart.as<int>(), ngroups, g.nbc, g.nsbc, g.igroup, g.bin_rows, g.bin_cols, g.w,
+        g.fp32 ? 16 : 8, g.nrows, g.nf2, g.row_wrap, d.ipts.as<double2>(), d.iperm.as<int>());
+    PF_TRY(check_launch("deal_points_kernel"));
+    // the points' bin order is freed by the caller where only the interpolation needs it
+    PF_CUDA(cudaStreamSynchronize(s));
+    return 0;
+}
+
+// kernel width from which interpolation runs on the matrix instruction too: below it the
+// thread-per-point kernels are as fast or faster (lmax 1024, 511,063 points: 37 us against 44 at
+// w = 9, 50 against 52 at w = 10, but 63 against 54 at w = 11 and 140 against 84 at w = 16; 6 to 20
+// points per 100 grid cells: 33-37 against 27-31 at w = 11)
+constexpr int kMmaInterpWidth = 11;
+// points of an item and its most strips. Fewer points or strips make more and shorter items, which
+// pay for the edges of their windows but fill the GPU where there are few points: with strips
+// unbounded, spreading 10,000 points at lmax 1024 took 40 us, at most 8 strips 20, at most 4 22;
+// items of 16 points instead of 32 took 32 us instead of 25 for 100,003 points at lmax 511 (w = 11)
+constexpr int kMmaItemPoints = 32, kMmaItemStrips = 6;
+// slots past which a sparse set of points (over 8 slots to a point) keeps the bins' kernels: 1.6 GB
+constexpr int64_t kMmaMaxSlots = (int64_t)1 << 26;
+
+// The matrix-instruction kernels' slots: groups of up to 8 consecutive sorted points of one block
+// of columns that lie in at most two neighbouring strips, and the work items: stretches of
+// consecutive groups of one block, of about `want` points (several items per resident warp, so
+// that the last ones to end do not leave the GPU idle), padded to whole batches of 4 groups. Most
+// slots first.
+static int mma_slots(NufftGrid& g, NufftDev& d, const std::vector<int>& cnt, int nstrips, int nblocks,
+                     const double2* gg, const int* sidx, cudaStream_t s) {
+    const int want = (int)std::max<int64_t>(kMmaItemPoints, g.M / (148 * 24 * 3));
+    const int most = std::max(1, std::min(g.item_rows / 4, kMmaItemStrips)), far = mma_max_advance();
+    std::vector<int4> items;
+    std::vector<MmaGroup> groups;
+    groups.reserve(g.M / 7 + 16);
+    int p = 0;
+    for (int bc = 0; bc < nblocks; ++bc) {
+        const int* c = cnt.data() + (size_t)bc * nstrips;
+        const int col = bc * g.blk_cols;
+        int first = -1, first_group = 0, have = 0, last = 0;  // the open item; its last group's strip
+        auto close = [&] {
+            if (first < 0) return;
+            while ((groups.size() - first_group) % 4) groups.push_back(MmaGroup{0, 0, last, col, 0});
+            items.push_back(make_int4(4 * first, col, 8 * first_group, 8 * (int)groups.size()));
+            first = -1;
+            have = 0;
+        };
+        int left = 0;  // points of strip br not yet in a group
+        for (int br = 0; br < nstrips; ++br) {
+            left += c[br];
+            while (left > 0) {
+                // a group starting in strip br, with points of strip br + 1 if br has under 8 left
+                if (first >= 0 && (have >= want || br - first >= most || br - last > far)) close();
+                if (first < 0) {
+                    first = last = br;
+                    first_group = (int)groups.size();
+                }
+                int n = std::min(left, 8);
+                left -= n;
+                if (n < 8 && br + 1 < nstrips) {
+                    const int more = std::min(8 - n, c[br + 1]);
+                    n += more;
+                    left -= more;  // taken from the next strip's count
+                }
+                groups.push_back(MmaGroup{p, n, br, col, br - last});
+                last = br;
+                p += n;
+                have += n;
+            }
+        }
+        close();
+    }
+    const int64_t nslots = 8 * (int64_t)groups.size();
+    g.nitems = 0;
+    if (nslots > kMmaMaxSlots && nslots > 8 * g.M) return 0;
+    std::stable_sort(items.begin(), items.end(), [](const int4& a, const int4& b) { return a.w - a.z > b.w - b.z; });
+    g.nitems = (int)items.size();
+    if (p != g.M || nslots > INT32_MAX) {
+        set_error("grouping the NUFFT points failed");
+        return 1;
+    }
+    DevBuf dg;
+    PF_TRY(dg.alloc(sizeof(MmaGroup) * std::max<size_t>(groups.size(), 1)));
+    PF_TRY(d.items.alloc(sizeof(int4) * std::max<size_t>(items.size(), 1)));
+    PF_TRY(d.soff.alloc(sizeof(double2) * std::max<int64_t>(nslots, 1)));
+    PF_TRY(d.smeta.alloc(sizeof(int2) * std::max<int64_t>(nslots, 1)));
+    if (nslots > 0) {
+        PF_CUDA(cudaMemcpyAsync(dg.p, groups.data(), sizeof(MmaGroup) * groups.size(), cudaMemcpyHostToDevice, s));
+        PF_CUDA(cudaMemcpyAsync(d.items.p, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, s));
+        PF_TRY(mma_fill_slots(g, d, gg, sidx, dg.as<MmaGroup>(), nslots, s));
+    }
+    PF_CUDA(cudaStreamSynchronize(s));
+    return 0;
+}
+
+// the points sorted by bins (or strips) of br x bc origin cells: grid coordinates in gg, the sorted
+// order in sidx, the points per bin in counts
+static int sort_points(const NufftGrid& g, const double* x, const double* y, int rows, int cols, int nbr,
+                       int nbc, int strips, DevBuf& gg, DevBuf& sidx, DevBuf& counts, cudaStream_t s) {
+    const int64_t M = g.M;
+    const int64_t nbins = (int64_t)nbr * nbc, nkeys = nbins * rows * cols;
+    if (nkeys > INT32_MAX) {
+        set_error("NUFFT fine grid too large for 32-bit bin keys");
+        return 1;
+    }
+    DevBuf key, key2, idx, tmp;
+    PF_TRY(gg.alloc(sizeof(double2) * M));
+    PF_TRY(key.alloc(sizeof(int) * M));
+    PF_TRY(key2.alloc(sizeof(int) * M));
+    PF_TRY(idx.alloc(sizeof(int) * M));
+    PF_TRY(sidx.alloc(sizeof(int) * M));
+    PF_TRY(counts.alloc(sizeof(int) * (nbins + 1)));
+    PF_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * (nbins + 1), s));
+    const double s1 = (double)g.nf1 / (2 * M_PI), s2 = (double)g.nf2 / (2 * M_PI);
+    bin_keys_kernel<<<nblk(M, 256), 256, 0, s>>>(x, y, M, s1, s2, g.row0, g.row_wrap, g.nf1, g.nf2, g.nrows,
+                                                 g.w, rows, cols, nbr, nbc, strips, gg.as<double2>(),
+                                                 key.as<int>(), idx.as<int>(), counts.as<int>());
+    PF_TRY(check_launch("bin_keys_kernel"));
+    int end_bit = 1;
+    while ((1ll << end_bit) < nkeys && end_bit < 31) ++end_bit;
+    size_t tb = 0;
+    PF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.as<int>(), key2.as<int>(), idx.as<int>(),
+                                            sidx.as<int>(), (int)M, 0, end_bit, s));
+    PF_TRY(tmp.alloc(tb));
+    PF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.as<int>(), key2.as<int>(), idx.as<int>(),
+                                            sidx.as<int>(), (int)M, 0, end_bit, s));
+    // temporaries are freed when this returns, so finish using them first
+    PF_CUDA(cudaStreamSynchronize(s));
+    return 0;
+}
+
+static int host_counts(const DevBuf& counts, int64_t n, std::vector<int>& cnt, cudaStream_t s) {
+    cnt.resize(n);
+    PF_CUDA(cudaMemcpyAsync(cnt.data(), counts.p, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
     PF_CUDA(cudaStreamSynchronize(s));
     return 0;
 }
@@ -270,104 +403,96 @@ int nufft_setpts(NufftGrid& g, NufftDev& d, const double* x, const double* y, cu
         set_error("more than 2^31-1 points in one plan");
         return 1;
     }
+    DevBuf gg, sidx, counts;
+    std::vector<int> cnt;
+    const int nstrips = (g.nrows + 3) / 4, nblocks = (g.nf2 + g.blk_cols - 1) / g.blk_cols;
+    // (grids of over 2^31 cells in strips, or 2^26 strips, keep the bins)
+    if ((int64_t)nstrips * nblocks > (1 << 26) || (int64_t)nstrips * nblocks * 4 * g.blk_cols > INT32_MAX) g.mma = 0;
+    if (g.mma) {
+        PF_TRY(sort_points(g, x, y, 4, g.blk_cols, nstrips, nblocks, 1, gg, sidx, counts, s));
+        PF_TRY(host_counts(counts, (int64_t)nstrips * nblocks, cnt, s));
+        PF_TRY(mma_slots(g, d, cnt, nstrips, nblocks, gg.as<double2>(), sidx.as<int>(), s));
+        g.mma = g.nitems > 0 ? 1 : 0;
+        g.mma_interp = g.mma && g.w >= kMmaInterpWidth ? 1 : 0;
+        if (g.mma_interp) return 0;
+    }
     g.nbr = std::max(1, (g.nrows + g.bin_rows - 1) / g.bin_rows);
     g.nbc = std::max(1, (g.nf2 + g.bin_cols - 1) / g.bin_cols);
     const int nbins = g.nbr * g.nbc;
-    DevBuf gg, key, key2, idx, idx2, counts, tmp;
-    PF_TRY(gg.alloc(sizeof(double2) * M));
-    PF_TRY(key.alloc(sizeof(int) * M));
-    PF_TRY(key2.alloc(sizeof(int) * M));
-    PF_TRY(idx.alloc(sizeof(int) * M));
-    PF_TRY(idx2.alloc(sizeof(int) * M));
-    PF_TRY(counts.alloc(sizeof(int) * (nbins + 1)));
+    PF_TRY(sort_points(g, x, y, g.bin_rows, g.bin_cols, g.nbr, g.nbc, 0, gg, sidx, counts, s));
     PF_TRY(d.binstart.alloc(sizeof(int) * (nbins + 1)));
-    PF_TRY(d.pts.alloc(sizeof(double2) * M));
-    PF_TRY(d.perm.alloc(sizeof(int) * M));
-    PF_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int) * (nbins + 1), s));
-    const double s1 = (double)g.nf1 / (2 * M_PI), s2 = (double)g.nf2 / (2 * M_PI);
-    bin_keys_kernel<<<nblk(M, 256), 256, 0, s>>>(x, y, M, s1, s2, g.row0, g.row_wrap, g.nf1,
-                                                 g.nf2, g.nrows, g.w, g.bin_rows, g.bin_cols,
-                                                 g.nbr, g.nbc,
-                                                 gg.as<double2>(), key.as<int>(), idx.as<int>(),
-                                                 counts.as<int>());
-    PF_TRY(check_launch("bin_keys_kernel"));
-    const int64_t nkeys = (int64_t)nbins * g.bin_rows * g.bin_cols;
-    if (nkeys > INT32_MAX) {
-        set_error("NUFFT fine grid too large for 32-bit bin keys");
-        return 1;
-    }
-    int end_bit = 1;
-    while ((1ll << end_bit) < nkeys && end_bit < 31) ++end_bit;
-    size_t tb = 0, tb2 = 0;
-    PF_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, key.as<int>(), key2.as<int>(),
-                                            idx.as<int>(), idx2.as<int>(), (int)M, 0, end_bit, s));
-    PF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, counts.as<int>(), d.binstart.as<int>(),
-                                          nbins + 1, s));
-    PF_TRY(tmp.alloc(std::max(tb, tb2)));
-    PF_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, key.as<int>(), key2.as<int>(),
-                                            idx.as<int>(), idx2.as<int>(), (int)M, 0, end_bit, s));
-    PF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb2, counts.as<int>(), d.binstart.as<int>(),
-                                          nbins + 1, s));
-    gather_points_kernel<<<nblk(M, 256), 256, 0, s>>>(gg.as<double2>(), idx2.as<int>(), M,
-                                                      d.pts.as<double2>(), d.perm.as<int>());
-    PF_TRY(check_launch("gather_points_kernel"));
-    // launch order of the bins: non-empty bins, most points first, so the heavy bins start
-    // in the first wave and the tail of the grid is the light ones
-    std::vector<int> cnt(nbins);
-    PF_CUDA(cudaMemcpyAsync(cnt.data(), counts.p, sizeof(int) * nbins, cudaMemcpyDeviceToHost, s));
-    // temporaries are freed when this returns, so finish using them first
-    PF_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> order;
-    order.reserve(nbins);
-    for (int b = 0; b < nbins; ++b)
-        if (cnt[b] > 0) order.push_back(b);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cnt[a] > cnt[b]; });
-    g.nbusy = (int)order.size();
-    PF_TRY(d.binorder.alloc(sizeof(int) * std::max<size_t>(order.size(), 1)));
-    if (!order.empty())
-        PF_CUDA(cudaMemcpyAsync(d.binorder.p, order.data(), sizeof(int) * order.size(),
-                                cudaMemcpyHostToDevice, s));
-    // spreading colours: tiles of bins rcol rows or ccol columns of bins apart are disjoint when
-    // the kernel's reach w - 1 fits in (rcol - 1) bins. Tiles that run past the grid's last column
-    // (or, when rows wrap, its last row) wrap onto its first ones, so those bins get colour
-    // classes of their own, one set for column wrap, one for row wrap and one for both; within
-    // such a set no two bins of one class both wrap, so their tiles stay disjoint as well.
+    // the points in bin order, for the spreading and to deal the interpolation's
+    DevBuf only_dealt_pts, only_dealt_perm;
+    DevBuf& pts = g.mma ? only_dealt_pts : d.pts;
+    DevBuf& perm = g.mma ? only_dealt_perm : d.perm;
+    PF_TRY(pts.alloc(sizeof(double2) * M));
+    PF_TRY(perm.alloc(sizeof(int) * M));
     {
-        const int rcol = 1 + (g.w - 1 + g.bin_rows - 1) / g.bin_rows;
-        const int ccol = 1 + (g.w - 1 + g.bin_cols - 1) / g.bin_cols;
-        const int K = rcol * ccol;
-        g.ncolors = 4 * K;
-        std::vector<int> sord;
-        g.color_off.assign(1, 0);
-        auto colour = [&](int b) {
-            const int br = b / g.nbc, bc = b % g.nbc;
-            const int cw = bc * g.bin_cols + g.bin_cols + g.w - 1 > g.nf2 ? 1 : 0;
-            const int rw = g.row_wrap && br * g.bin_rows + g.bin_rows + g.w - 1 > g.nrows ? 1 : 0;
-            return (br % rcol) * ccol + bc % ccol + K * (cw + 2 * rw);
-        };
-        for (int k = 0; k < g.ncolors; ++k) {
-            for (int b : order)
-                if (colour(b) == k) sord.push_back(b);
-            g.color_off.push_back((int)sord.size());
-        }
-        PF_TRY(d.sorder.alloc(sizeof(int) * std::max<size_t>(sord.size(), 1)));
-        if (!sord.empty())
-            PF_CUDA(cudaMemcpyAsync(d.sorder.p, sord.data(), sizeof(int) * sord.size(),
+        DevBuf tmp;
+        size_t tb = 0;
+        PF_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts.as<int>(), d.binstart.as<int>(), nbins + 1, s));
+        PF_TRY(tmp.alloc(tb));
+        PF_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tb, counts.as<int>(), d.binstart.as<int>(), nbins + 1, s));
+        gather_points_kernel<<<nblk(M, 256), 256, 0, s>>>(gg.as<double2>(), sidx.as<int>(), M,
+                                                          pts.as<double2>(), perm.as<int>());
+        PF_TRY(check_launch("gather_points_kernel"));
+        PF_TRY(host_counts(counts, nbins, cnt, s));
+    }
+    if (!g.mma) {
+        // launch order of the bins: non-empty bins, most points first, so the heavy bins start
+        // in the first wave and the tail of the grid is the light ones
+        std::vector<int> order;
+        order.reserve(nbins);
+        for (int b = 0; b < nbins; ++b)
+            if (cnt[b] > 0) order.push_back(b);
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cnt[a] > cnt[b]; });
+        g.nbusy = (int)order.size();
+        PF_TRY(d.binorder.alloc(sizeof(int) * std::max<size_t>(order.size(), 1)));
+        if (!order.empty())
+            PF_CUDA(cudaMemcpyAsync(d.binorder.p, order.data(), sizeof(int) * order.size(),
                                     cudaMemcpyHostToDevice, s));
-        // the register-tile spreading reads a bin's number and point range in one load
-        std::vector<int> first(nbins + 1, 0);
-        for (int b = 0; b < nbins; ++b) first[b + 1] = first[b] + cnt[b];
-        auto slots = [&](const std::vector<int>& ord, DevBuf& out) -> int {
-            std::vector<int4> v(std::max<size_t>(ord.size(), 1), make_int4(0, 0, 0, 0));
-            for (size_t i = 0; i < ord.size(); ++i)
-                v[i] = make_int4(ord[i], first[ord[i]], first[ord[i] + 1], 0);
-            PF_TRY(out.alloc(sizeof(int4) * v.size()));
-            PF_CUDA(cudaMemcpyAsync(out.p, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice, s));
-            PF_CUDA(cudaStreamSynchronize(s));
-            return 0;
-        };
-        PF_TRY(slots(order, d.bslot));
-        PF_TRY(slots(sord, d.sslot));
+        // spreading colours: tiles of bins rcol rows or ccol columns of bins apart are disjoint when
+        // the kernel's reach w - 1 fits in (rcol - 1) bins. Tiles that run past the grid's last column
+        // (or, when rows wrap, its last row) wrap onto its first ones, so those bins get colour
+        // classes of their own, one set for column wrap, one for row wrap and one for both; within
+        // such a set no two bins of one class both wrap, so their tiles stay disjoint as well.
+        {
+            const int rcol = 1 + (g.w - 1 + g.bin_rows - 1) / g.bin_rows;
+            const int ccol = 1 + (g.w - 1 + g.bin_cols - 1) / g.bin_cols;
+            const int K = rcol * ccol;
+            g.ncolors = 4 * K;
+            std::vector<int> sord;
+            g.color_off.assign(1, 0);
+            auto colour = [&](int b) {
+                const int br = b / g.nbc, bc = b % g.nbc;
+                const int cw = bc * g.bin_cols + g.bin_cols + g.w - 1 > g.nf2 ? 1 : 0;
+                const int rw = g.row_wrap && br * g.bin_rows + g.bin_rows + g.w - 1 > g.nrows ? 1 : 0;
+                return (br % rcol) * ccol + bc % ccol + K * (cw + 2 * rw);
+            };
+            for (int k = 0; k < g.ncolors; ++k) {
+                for (int b : order)
+                    if (colour(b) == k) sord.push_back(b);
+                g.color_off.push_back((int)sord.size());
+            }
+            PF_TRY(d.sorder.alloc(sizeof(int) * std::max<size_t>(sord.size(), 1)));
+            if (!sord.empty())
+                PF_CUDA(cudaMemcpyAsync(d.sorder.p, sord.data(), sizeof(int) * sord.size(),
+                                        cudaMemcpyHostToDevice, s));
+            // the register-tile spreading reads a bin's number and point range in one load
+            std::vector<int> first(nbins + 1, 0);
+            for (int b = 0; b < nbins; ++b) first[b + 1] = first[b] + cnt[b];
+            auto slots = [&](const std::vector<int>& ord, DevBuf& out) -> int {
+                std::vector<int4> v(std::max<size_t>(ord.size(), 1), make_int4(0, 0, 0, 0));
+                for (size_t i = 0; i < ord.size(); ++i)
+                    v[i] = make_int4(ord[i], first[ord[i]], first[ord[i] + 1], 0);
+                PF_TRY(out.alloc(sizeof(int4) * v.size()));
+                PF_CUDA(cudaMemcpyAsync(out.p, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice, s));
+                PF_CUDA(cudaStreamSynchronize(s));
+                return 0;
+            };
+            PF_TRY(slots(order, d.bslot));
+            PF_TRY(slots(sord, d.sslot));
+        }
     }
     // interpolation groups igroup consecutive bins of a bin row; non-empty groups, most
     // points first
@@ -385,7 +510,7 @@ int nufft_setpts(NufftGrid& g, NufftDev& d, const double* x, const double* y, cu
         PF_CUDA(cudaMemcpyAsync(d.iorder.p, gorder.data(), sizeof(int) * gorder.size(),
                                 cudaMemcpyHostToDevice, s));
     PF_CUDA(cudaStreamSynchronize(s));
-    return interp_point_order(g, d, binstart_host(g, d, s), s);
+    return interp_point_order(g, d, pts.as<double2>(), perm.as<int>(), s);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -507,21 +632,6 @@ static int fine_fft(cufftHandle h, void* data, bool fp32, int dir) {
                               static_cast<cufftDoubleComplex*>(data), dir));
     return 0;
 }
-
-// ---------------------------------------------------------------------------------------
-// complex element of the fine grids: double2 in the FP64 form, float2 in the mixed form (whose
-// mode columns, points and per-mode factors stay FP64)
-// ---------------------------------------------------------------------------------------
-template <class T> struct Cx;
-template <> struct Cx<double> {
-    using t = double2;
-    __device__ static double2 make(double x, double y) { return make_double2(x, y); }
-};
-template <> struct Cx<float> {
-    using t = float2;
-    __device__ static float2 make(float x, float y) { return make_float2(x, y); }
-};
-template <class T> using cx = typename Cx<T>::t;
 
 // ---------------------------------------------------------------------------------------
 // pad / unpad along dim 1
@@ -786,99 +896,6 @@ int make_tile_map(CUtensorMap* map, void* base, int esize, int64_t inner, int64_
 // ---------------------------------------------------------------------------------------
 // interpolation and spreading
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ int wrap(int i, int n) {
-    int r = i % n;
-    return r < 0 ? r + n : r;
-}
-
-// tile of a bin: the rows and columns its points' kernels reach,
-// rows [br BR, br BR + BR + W - 1) x columns [bc BC, bc BC + BC + W - 1)
-struct TileGeom {
-    int tr0, tc0, TR, TC;
-};
-template <int W>
-__device__ __forceinline__ TileGeom tile_geom(int bin, int nbc, int BR, int BC) {
-    const int br = bin / nbc, bc = bin % nbc;
-    return TileGeom{br * BR, bc * BC, BR + W - 1, BC + W - 1};
-}
-
-// origin cell of a point inside its bin's tile (the binning of bin_keys_kernel)
-template <int W>
-__device__ __forceinline__ void local_origin(double2 g, const TileGeom& tg, int nrows, int nf2,
-                                             int row_wrap, int& r0, int& c0, double& v1,
-                                             double& v2) {
-    const int i10 = (int)ceil(g.x - 0.5 * W);
-    const int i20 = (int)ceil(g.y - 0.5 * W);
-    v1 = ((double)i10 - g.x) + (0.5 * W - 0.5);
-    v2 = ((double)i20 - g.y) + (0.5 * W - 0.5);
-    int r = i10, c = i20;
-    if (row_wrap) r = wrap(r, nrows);
-    c = wrap(c, nf2);
-    r0 = r - tg.tr0;
-    c0 = c - tg.tc0;
-}
-
-template <int W, class T> struct EsCoef;
-template <int W> struct EsCoef<W, double> {
-    __device__ static const double* get() { return EsHorner<W>::coef(); }
-};
-template <int W> struct EsCoef<W, float> {
-    __device__ static const float* get() { return EsHorner<W>::coef_f(); }
-};
-
-// Weights of the mirrored taps a and W - 1 - a (a < W / 2) at offset v, u = v^2, in the grid's
-// precision. Tap W - 1 - a is tap a reflected (v -> -v; the table holds the same coefficients
-// with the odd powers negated), so with p_a(v) = E(v^2) + v O(v^2) the pair costs one even and
-// one odd Horner chain in u: NC multiply-adds for two taps instead of 2 (NC - 1).
-template <int W, class T>
-__device__ __forceinline__ void es_pair(int a, T v, T u, T& ka, T& kb) {
-    constexpr int NC = EsHorner<W>::NC;
-    constexpr int NE = (NC + 1) / 2, NO = NC / 2;
-    const T* cf = EsCoef<W, T>::get() + a * NC;
-    T e = cf[2 * (NE - 1)];
-#pragma unroll
-    for (int i = NE - 2; i >= 0; --i) e = fma(e, u, cf[2 * i]);
-    T o = cf[2 * (NO - 1) + 1];
-#pragma unroll
-    for (int i = NO - 2; i >= 0; --i) o = fma(o, u, cf[2 * i + 1]);
-    ka = fma(v, o, e);
-    kb = fma(-v, o, e);
-}
-
-// weight of the middle tap of an odd width (an even polynomial: its odd coefficients are 0)
-template <int W, class T>
-__device__ __forceinline__ T es_mid(T u) {
-    constexpr int NC = EsHorner<W>::NC;
-    constexpr int NE = (NC + 1) / 2;
-    const T* cf = EsCoef<W, T>::get() + (W / 2) * NC;
-    T e = cf[2 * (NE - 1)];
-#pragma unroll
-    for (int i = NE - 2; i >= 0; --i) e = fma(e, u, cf[2 * i]);
-    return e;
-}
-
-// all W tap weights at offset v: mirrored pairs in FP64; one Horner chain per tap in FP32, where
-// the spreading kernel measured faster that way (0.133 vs 0.142 ms at lmax 2048)
-template <int W, class T>
-__device__ __forceinline__ void es_weights(T v, T (&k)[W]) {
-    if constexpr (sizeof(T) == 8) {
-        const T u = v * v;
-#pragma unroll
-        for (int a = 0; a < W / 2; ++a) es_pair<W, T>(a, v, u, k[a], k[W - 1 - a]);
-        if constexpr (W & 1) k[W / 2] = es_mid<W, T>(u);
-    } else {
-        constexpr int NC = EsHorner<W>::NC;
-        const T* cf = EsCoef<W, T>::get();
-#pragma unroll
-        for (int a = 0; a < W; ++a) {
-            T p = cf[a * NC + NC - 1];
-#pragma unroll
-            for (int q = NC - 2; q >= 0; --q) p = fma(p, v, cf[a * NC + q]);
-            k[a] = p;
-        }
-    }
-}
-
 // one point's interpolation from its group's tile (rows TS elements apart): the w x w taps,
 // rows in mirrored pairs with the column weights held in registers; 0 for a point outside the
 // tile (which binning excludes)
@@ -1756,6 +1773,7 @@ static int launch_spread(const NufftGrid& g, NufftDev& d, const double2* f, int 
 
 template <class T>
 static int interp_any(const NufftGrid& g, NufftDev& d, double2* f, int B, cudaStream_t s) {
+    if (g.mma_interp) return interp_mma(g, d, f, B, s);
 #define PF_CALL(WW) launch_interp<WW, T>(g, d, f, B, s)
     PF_WIDTH_SWITCH(PF_CALL)
 #undef PF_CALL
@@ -1763,6 +1781,7 @@ static int interp_any(const NufftGrid& g, NufftDev& d, double2* f, int B, cudaSt
 
 template <class T>
 static int spread_any(const NufftGrid& g, NufftDev& d, const double2* f, int B, cudaStream_t s) {
+    if (g.mma) return spread_mma(g, d, f, B, s);
 #define PF_CALL(WW) launch_spread<WW, T>(g, d, f, B, s)
     PF_WIDTH_SWITCH(PF_CALL)
 #undef PF_CALL

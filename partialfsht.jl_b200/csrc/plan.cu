@@ -99,6 +99,12 @@ int setup_nufft_grid(NufftGrid& g, NufftDev& d, int n1, int nmodes2, const std::
     if (bin_cols > 0 && bin_cols < g.bin_cols) g.bin_cols = bin_cols;
     // interpolation tiles of up to 32 columns: as many whole bins as fit
     g.igroup = std::max(1, (33 - g.w) / g.bin_cols);
+    // FP64 grids spread on the matrix instruction (the deterministic option's colour launches and
+    // the window option keep their own kernels)
+    g.mma = !fp32 && !g.deterministic && g.spread_reg ? 1 : 0;
+    g.blk_cols = mma_tile_cols(g.w) + 1 - g.w;
+    if (bin_cols > 0 && bin_cols < g.blk_cols) g.blk_cols = bin_cols;
+    g.item_rows = bin_rows > 0 ? bin_rows : 1 << 20;
     if (full_rows) {
         g.row0 = 0;
         g.nrows = g.nf1;
@@ -218,7 +224,7 @@ void fill_info(pfsht_plan* p) {
                             &p->adj_seg.ck_p, &p->adj_seg.ck_E,
                             &p->H, &p->phi_pts, &p->nd.pts, &p->nd.perm, &p->nd.binstart,
                             &p->nd.binorder, &p->nd.sorder, &p->nd.bslot, &p->nd.sslot,
-                            &p->nd.iorder, &p->nd.ipts, &p->nd.iperm, &p->nd.counter,
+                            &p->nd.iorder, &p->nd.items, &p->nd.soff, &p->nd.smeta, &p->nd.ipts, &p->nd.iperm, &p->nd.counter,
                             &p->nd.colp2, &p->nd.p2col, &p->nd.mult1, &p->nd.dec2, &p->nd.pad,
                             &p->nd.U, &p->st_alm, &p->st_f, &p->ab_fwd, &p->st_alm2,
                             &p->st_f2, &p->blk_fwd_items, &p->blk_adj_items})
@@ -382,14 +388,14 @@ int build_stretch(pfsht_plan* p, const double* d_theta, const double* d_phi, con
     }
     std::vector<int> colk2(p->ncols);
     for (int c = 0; c < p->ncols; ++c) colk2[c] = c - lf.mmax;
+    p->ng.plain_transpose = o.nufft_transpose == 1 ? 1 : 0;
+    p->ng.spread_reg = o.nufft_spread == 1 ? 0 : 1;
+    p->ng.deterministic = p->deterministic;
     PF_TRY(setup_nufft_grid(p->ng, p->nd, lf.nth, lf.nph, colk2, phase, p->tol, p->M, Tmin, Tmax,
                             false, o.nufft_bin_rows, o.nufft_bin_cols,
                             p->precision == PFSHT_PRECISION_MIXED, o.nufft_fft_lengths, o.nufft_nf1,
                             o.nufft_nf2, s));
     PF_TRY(nufft_setpts(p->ng, p->nd, Th.as<double>(), ph.as<double>(), s));
-    p->ng.plain_transpose = o.nufft_transpose == 1 ? 1 : 0;
-    p->ng.spread_reg = o.nufft_spread == 1 ? 0 : 1;
-    p->ng.deterministic = p->deterministic;
     PF_TRY(nufft_alloc(p->ng, p->nd, B));
     return 0;
 }
