@@ -128,10 +128,17 @@ struct RingItems {
     const unsigned char* sole_m = nullptr; // lmax + 1: order covered by a single tile
     const int* jlo = nullptr;              // lmax + 1 retained ring range
     const int* jhi = nullptr;
+    // the forward's items in blocks of kFwdBlockItems, an order's degrees split over the warps of a
+    // block where that is worth it (RingItem::pad_ = split_code); null: one warp per item
+    const RingItem* blocks = nullptr;
+    int nblocks = 0, block_rmax = 4;
 };
+constexpr int kFwdBlockItems = 4;
+// warps that share an item's rings, each a piece of its degrees, and this one's place among them
+__host__ __device__ constexpr int split_code(int size, int place) { return size | place << 8; }
 
 struct RingItemsOwner {
-    DevBuf items, sole, jlo, jhi;
+    DevBuf items, sole, jlo, jhi, blocks;
     RingItems view;
     std::vector<RingItem> host;  // the items, in launch order
 };
@@ -199,12 +206,20 @@ std::vector<RingItem> make_ring_items(const std::vector<int>& jlo, const std::ve
 int build_ring_items(const std::vector<int>& jlo, const std::vector<int>& jhi, int lmax, int mmax,
                      int rmax, RingItemsOwner& own, cudaStream_t s,
                      const RingSegments* seg = nullptr, int tile = 0);
-// choose the degree segments for a ring set (seg_degrees > 0: target length; 0: none) and
+// the forward's blocks over tiles of 32 rmax rings, split along the degrees by `seg` (at most
+// kFwdBlockItems segments per order)
+std::vector<RingItem> make_fwd_blocks(const std::vector<int>& jlo, const std::vector<int>& jhi, int lmax,
+                                      int mmax, int tile, const RingSegments& seg, const std::vector<int>& bounds,
+                                      std::vector<int>& off);
+int build_fwd_blocks(const std::vector<int>& jlo, const std::vector<int>& jhi, int lmax, int mmax,
+                     int rmax, const RingSegments& seg, RingItemsOwner& own, cudaStream_t s);
+// choose the degree segments for a ring set (seg_degrees > 0: target length, at most max_segs per
+// order; 0: none) and
 // save the recurrence state at every segment start; t.ab/aboff must be built. Returns the
 // segments unused (nseg all 1) when the state would exceed max_bytes.
 int build_ring_segments(const RingTables& t, const std::vector<int>& jlo,
                         const std::vector<int>& jhi, int lmax, int mmax, int seg_degrees,
-                        int64_t max_bytes, RingSegments& seg, cudaStream_t s);
+                        int64_t max_bytes, RingSegments& seg, cudaStream_t s, int max_segs = 1 << 20);
 // launchers: B transforms, alm complex (lmax+1, 2lmax+1, B); the adjoint writes all of alm
 int ring_forward(const RingTables& t, const RingOut& o, const RingItems& it, const double2* alm,
                  double2* out, int B, cudaStream_t s);

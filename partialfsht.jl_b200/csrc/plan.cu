@@ -221,7 +221,7 @@ void fill_info(pfsht_plan* p) {
     }
     int64_t bytes = 0;
     for (const DevBuf* b : {&p->cos_t, &p->log2sin, &p->log2c, &p->w, &p->ab, &p->aboff, &p->fwd_items.items, &p->adj_items.items,
-                            &p->adj_seg.ck_p, &p->adj_seg.ck_E,
+                            &p->adj_seg.ck_p, &p->adj_seg.ck_E, &p->fwd_seg.ck_p, &p->fwd_seg.ck_E, &p->fwd_items.blocks,
                             &p->H, &p->phi_pts, &p->nd.pts, &p->nd.perm, &p->nd.binstart,
                             &p->nd.binorder, &p->nd.sorder, &p->nd.bslot, &p->nd.sslot,
                             &p->nd.iorder, &p->nd.items, &p->nd.soff, &p->nd.smeta, &p->nd.ipts, &p->nd.iperm, &p->nd.counter,
@@ -313,6 +313,26 @@ int build_adjoint_items(pfsht_plan* p, const std::vector<int>& jlo, const std::v
                             p->adj_seg.seg_degrees > 0 ? &p->adj_seg : nullptr, tile);
 }
 
+// The forward's blocks: each (order, tile of rings) split into up to four pieces of at least 64
+// degrees, one per warp of a block, unless there are items enough for many waves. A plan has only a
+// few thousand items of very different lengths, so whole items left the GPU part idle behind the
+// longest ones, and in small plans one item's chain of degrees was the pass.
+constexpr int kFwdWholeItems = 148 * 20 * 8;
+// rings per lane of the forward: a degree's coefficients cost five shared-memory wavefronts whatever
+// the rings, so four rings a lane halve that traffic for one transform (lmax 2048: 177 us against 192
+// with two, lmax 1024 45 against 49, lmax 256 12 against 16); several transforms share the coefficients'
+// recurrence loads anyway and two rings keep their accumulators in registers (lmax 1024, two
+// transforms: 67 us against 76)
+int fwd_rings(const pfsht_plan* p) { return p->R > 0 ? p->R : p->B == 1 ? 4 : 2; }
+int build_forward_blocks(pfsht_plan* p, const std::vector<int>& jlo, const std::vector<int>& jhi, int mmax,
+                         cudaStream_t s) {
+    if (p->fwd_items.view.nitems >= kFwdWholeItems) return 0;
+    PF_TRY(build_ring_segments(p->rt_fwd, jlo, jhi, p->L, mmax, 64, (int64_t)512 << 20, p->fwd_seg, s, kFwdBlockItems));
+    p->rt_fwd.ck_p = p->fwd_seg.ck_p.as<double2>();
+    p->rt_fwd.ck_E = p->fwd_seg.ck_E.as<int>();
+    return build_fwd_blocks(jlo, jhi, p->L, mmax, fwd_rings(p), p->fwd_seg, p->fwd_items, s);
+}
+
 int build_stretch(pfsht_plan* p, const double* d_theta, const double* d_phi, const pfsht_opts& o,
                   cudaStream_t s) {
     Leaf& lf = p->leaf;
@@ -341,9 +361,9 @@ int build_stretch(pfsht_plan* p, const double* d_theta, const double* d_phi, con
         p->rt.aboff = p->aboff.as<int64_t>();
         p->rt.lmax = L;
         p->rt.nrings = lf.nth_half;
-        // forward tiles of 64 rings in the FP64 form (more warps) and of 128 in the mixed form
-        // (measured faster), adjoint tiles of 128 (amortises its reduction), split along the
-        // degree axis when the tiles alone leave the GPU under-filled
+        // forward tiles of 128 rings (64 with several transforms, fwd_rings; 64 in a batch, whose
+        // warps pull whole items), adjoint tiles of 128 (amortises its reduction), both split along
+        // the degree axis when the tiles alone leave the GPU under-filled
         p->rt_fwd = p->rt;
         if (mix) {
             DevBuf off_unused;  // the offsets equal p->aboff (they depend on lmax and mmax only)
@@ -353,6 +373,7 @@ int build_stretch(pfsht_plan* p, const double* d_theta, const double* d_phi, con
             p->rt_fwd.stride = 64;
         }
         PF_TRY(build_ring_items(lf.jlo, lf.jhi, L, lf.mmax, p->R > 0 ? p->R : 2, p->fwd_items, s));
+        PF_TRY(build_forward_blocks(p, lf.jlo, lf.jhi, lf.mmax, s));
         PF_TRY(build_adjoint_items(p, lf.jlo, lf.jhi, lf.mmax, s));
     }
     p->ncols = 2 * lf.mmax + 1;
@@ -440,6 +461,7 @@ int build_direct_rings(pfsht_plan* p, const double* h_theta, cudaStream_t s) {
     p->rt.nrings = (int)M;
     p->rt_fwd = p->rt;
     PF_TRY(build_ring_items(jlo, jhi, L, L, p->R > 0 ? p->R : 2, p->fwd_items, s));
+    if (!mix) PF_TRY(build_forward_blocks(p, jlo, jhi, L, s));
     return build_adjoint_items(p, jlo, jhi, L, s);
 }
 
@@ -1021,6 +1043,22 @@ static int group_items_by_block(pfsht_plan* p, const std::vector<RingItem>& item
     return 0;
 }
 
+// the forward's blocks grouped the same way (the same pieces of every order, so the same sums)
+static int group_fwd_blocks(pfsht_plan* p, const std::vector<AlmBlock>& blocks) {
+    std::vector<int> bounds;
+    for (const AlmBlock& k : blocks) bounds.push_back((k.c0 + 1) / 2);
+    bounds.push_back((blocks.back().c1 + 1) / 2);
+    const std::vector<RingItem> v = make_fwd_blocks(p->leaf.jlo, p->leaf.jhi, p->L, p->leaf.mmax,
+                                                    32 * p->fwd_items.view.block_rmax, p->fwd_seg, bounds,
+                                                    p->blk_fwd_off);
+    PF_TRY(p->blk_fwd_items.alloc(sizeof(RingItem) * std::max<size_t>(v.size(), 1)));
+    if (!v.empty())
+        PF_CUDA(cudaMemcpyAsync(p->blk_fwd_items.p, v.data(), sizeof(RingItem) * v.size(), cudaMemcpyHostToDevice,
+                                p->st_stream));
+    PF_CUDA(cudaStreamSynchronize(p->st_stream));
+    return 0;
+}
+
 int plan_host_staging(pfsht_plan* p) {
     const size_t na = sizeof(double2) * (size_t)(p->L + 1) * (2 * p->L + 1) * p->B;
     const size_t nf = sizeof(double2) * (size_t)p->M * p->B;
@@ -1040,7 +1078,8 @@ int plan_host_staging(pfsht_plan* p) {
     const bool blocked = p->kind != kDirect && p->kind != kMultiBox && p->spin == 0;
     if (blocked && !p->host_pipeline) {
         const std::vector<AlmBlock> blocks = alm_blocks(p->L, host_mmax(p));
-        PF_TRY(group_items_by_block(p, p->fwd_items.host, blocks, p->blk_fwd_items, p->blk_fwd_off));
+        if (p->fwd_items.view.blocks) PF_TRY(group_fwd_blocks(p, blocks));
+        else PF_TRY(group_items_by_block(p, p->fwd_items.host, blocks, p->blk_fwd_items, p->blk_fwd_off));
         PF_TRY(group_items_by_block(p, p->adj_items.host, blocks, p->blk_adj_items, p->blk_adj_off));
         p->ev_blk.assign(blocks.size(), nullptr);
         for (cudaEvent_t& e : p->ev_blk) PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1065,8 +1104,14 @@ static int host_forward_pipelined(pfsht_plan* p, const void* in, void* out, cuda
     for (size_t k = 0; k < blocks.size(); ++k) {
         PF_CUDA(cudaStreamWaitEvent(s, p->ev_blk[k], 0));
         RingItems v = p->fwd_items.view;
-        v.items = p->blk_fwd_items.as<RingItem>() + p->blk_fwd_off[k];
-        v.nitems = p->blk_fwd_off[k + 1] - p->blk_fwd_off[k];
+        const int n = p->blk_fwd_off[k + 1] - p->blk_fwd_off[k];
+        if (v.blocks) {
+            v.blocks = p->blk_fwd_items.as<RingItem>() + (int64_t)kFwdBlockItems * p->blk_fwd_off[k];
+            v.nblocks = n;
+        } else {
+            v.items = p->blk_fwd_items.as<RingItem>() + p->blk_fwd_off[k];
+            v.nitems = n;
+        }
         PF_TRY(ring_forward(p->rt_fwd, p->ro_cols, v, alm, p->H.as<double2>(), p->B, s));
     }
     clock_mark(&p->clk, kStRingFwd, s);

@@ -27,6 +27,7 @@ struct pfsht_plan {
     // ring pass
     DevBuf cos_t, log2sin, log2c, w, ab, aboff;
     RingItemsOwner fwd_items, adj_items;
+    RingSegments fwd_seg;  // degree segments of the forward's blocks
     RingSegments adj_seg;  // degree segments of the adjoint items
     int seg_degrees = 0;   // requested segment length (0 = auto, < 0 = none)
     RingTables rt;

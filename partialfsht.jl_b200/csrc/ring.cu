@@ -38,7 +38,7 @@
 
 namespace pf {
 
-static constexpr int kWarpsPerBlock = 4;  // forward
+static constexpr int kWarpsPerBlock = kFwdBlockItems;  // forward
 static constexpr int kAdjWarps = 1;       // adjoint (one-warp blocks: a finer tail)
 static constexpr int kAdjWarpsPersistent = 2;  // the batches' persistent adjoint (measured faster)
 
@@ -225,7 +225,7 @@ __global__ void ring_ckpt_kernel(RingTables t, const CkptJob* __restrict__ jobs,
 
 int build_ring_segments(const RingTables& t, const std::vector<int>& jlo,
                         const std::vector<int>& jhi, int L, int mmax, int seg_degrees,
-                        int64_t max_bytes, RingSegments& seg, cudaStream_t s) {
+                        int64_t max_bytes, RingSegments& seg, cudaStream_t s, int max_segs) {
     seg.nseg.assign(L + 1, 1);
     seg.nblk.assign(L + 1, 0);
     seg.ckbase.assign(L + 1, 0);
@@ -239,7 +239,7 @@ int build_ring_segments(const RingTables& t, const std::vector<int>& jlo,
         const int nret = jhi[m] - jlo[m] + 1;
         const int nb = L >= m + 2 ? (L - m - 1 + 63) / 64 : 0;
         seg.nblk[m] = nb;
-        const int K = std::max(1, std::min(nb, (nb + q / 2) / q));
+        const int K = std::max(1, std::min({nb, (nb + q / 2) / q, max_segs}));
         if (nret <= 0 || K <= 1) continue;
         seg.nseg[m] = K;
         seg.ckbase[m] = tot;
@@ -335,11 +335,17 @@ __device__ __forceinline__ CoefT<MIX> to_coef(double2 v) {
     else return v;
 }
 
+// one warp's part of its rings' sums where an order's degrees are split over the block's warps
+struct FwdPart {
+    double2 p[4][32], m[4][32];
+};
+
 template <int R, int NB, bool MIX>
 __device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut& o,
                                               const RingItem& item, const double2* __restrict__ alm,
                                               double2* __restrict__ out, int b0,
-                                              FwdSmem<NB, MIX>& sm, int warp, int lane) {
+                                              FwdSmem<NB, MIX>& sm, int warp, int lane,
+                                              FwdPart* parts, int size, int place) {
     constexpr int STRIDE = MIX ? 16 : 64;
     const int m = item.m, L = t.lmax;
     const double sgn = (m & 1) ? -1.0 : 1.0;
@@ -530,26 +536,67 @@ __device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut
     }
     // write the ring columns (window and 2^E folded into one exact scale)
     const double smir = o.spin_sgn * sgn;
+    auto write = [&](int k, int b, double2 gp, double2 gm) {
+        double2* ob = out + o.bstride * (b0 + b);
+        const int j = item.j0 + k;
+        ob[j + o.ld * (o.col_off + m)] = gp;
+        if (m > 0) ob[j + o.ld * (o.col_off - m)] = gm;
+        if (o.reflect) {
+            const int jj = o.nrows - 1 - j;
+            ob[jj + o.ld * (o.col_off + m)] = make_double2(gp.x * smir, gp.y * smir);
+            if (m > 0) ob[jj + o.ld * (o.col_off - m)] = make_double2(gm.x * smir, gm.y * smir);
+        }
+    };
+    double sc[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int k = lane + 32 * r;
-        if (k >= item.n) continue;
-        const int j = item.j0 + k;
-        const double sc = scalbn(t.w ? t.w[j] : 1.0, E[r]);
+        sc[r] = k < item.n ? scalbn(t.w ? t.w[item.j0 + k] : 1.0, E[r]) : 0.0;
+    }
+    if (size == 1) {
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            double2* ob = out + o.bstride * (b0 + b);
-            const double2 tp = accp[r][b].total(), tm = accm[r][b].total();
-            const double2 gp = make_double2(tp.x * sc, tp.y * sc);
-            const double2 gm = make_double2(tm.x * sc, tm.y * sc);
-            ob[j + o.ld * (o.col_off + m)] = gp;
-            if (m > 0) ob[j + o.ld * (o.col_off - m)] = gm;
-            if (o.reflect) {
-                const int jj = o.nrows - 1 - j;
-                ob[jj + o.ld * (o.col_off + m)] = make_double2(gp.x * smir, gp.y * smir);
-                if (m > 0) ob[jj + o.ld * (o.col_off - m)] = make_double2(gm.x * smir, gm.y * smir);
+        for (int r = 0; r < R; ++r) {
+            const int k = lane + 32 * r;
+            if (k >= item.n) continue;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const double2 tp = accp[r][b].total(), tm = accm[r][b].total();
+                write(k, b, make_double2(tp.x * sc[r], tp.y * sc[r]), make_double2(tm.x * sc[r], tm.y * sc[r]));
             }
         }
+        return;
+    }
+    // the degrees are split over `size` warps of the block: their parts are added in order
+    const int lead = warp - place;
+    auto meet = [&] {
+        if (size == kWarpsPerBlock) asm volatile("bar.sync 1, 128;" ::: "memory");
+        else if (lead == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+        else asm volatile("bar.sync 2, 64;" ::: "memory");
+    };
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const double2 tp = accp[r][b].total(), tm = accm[r][b].total();
+            parts[warp].p[r][lane] = make_double2(tp.x * sc[r], tp.y * sc[r]);
+            parts[warp].m[r][lane] = make_double2(tm.x * sc[r], tm.y * sc[r]);
+        }
+        meet();
+        for (int r = place; r < R; r += size) {
+            const int k = lane + 32 * r;
+            if (k < item.n) {
+                double2 gp = parts[lead].p[r][lane], gm = parts[lead].m[r][lane];
+                for (int q = 1; q < size; ++q) {
+                    const double2 up = parts[lead + q].p[r][lane], um = parts[lead + q].m[r][lane];
+                    gp.x += up.x;
+                    gp.y += up.y;
+                    gm.x += um.x;
+                    gm.y += um.y;
+                }
+                write(k, b, gp, gm);
+            }
+        }
+        meet();
     }
 }
 
@@ -581,7 +628,8 @@ __device__ __forceinline__ void ring_fwd_body(const RingTables& t, const RingOut
                                               const int* __restrict__ jhi,
                                               const double2* __restrict__ alm,
                                               double2* __restrict__ out, int b0,
-                                              FwdSmem<NB, MIX>& sm, int warp, int lane) {
+                                              FwdSmem<NB, MIX>& sm, int warp, int lane,
+                                              FwdPart* parts = nullptr, int size = 1, int place = 0) {
     if ((item.flags & kItemFirst) && o.zero_rest)
         ring_fwd_zero_rest<NB>(o, item, jlo[item.m], jhi[item.m], out, b0, lane);
     for (int base = 0; base < item.n; base += 32 * RMAX) {
@@ -590,9 +638,9 @@ __device__ __forceinline__ void ring_fwd_body(const RingTables& t, const RingOut
         sub.n = min(32 * RMAX, item.n - base);
         if (sub.ck >= 0) sub.ck += base;
         const int reff = (sub.n + 31) >> 5;
-        if (RMAX >= 4 && reff >= 3) ring_fwd_item<(RMAX >= 4 ? 4 : 1), NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane);
-        else if (RMAX >= 2 && reff == 2) ring_fwd_item<(RMAX >= 2 ? 2 : 1), NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane);
-        else ring_fwd_item<1, NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane);
+        if (RMAX >= 4 && reff >= 3) ring_fwd_item<(RMAX >= 4 ? 4 : 1), NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
+        else if (RMAX >= 2 && reff == 2) ring_fwd_item<(RMAX >= 2 ? 2 : 1), NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
+        else ring_fwd_item<1, NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
     }
 }
 
@@ -606,6 +654,21 @@ ring_fwd_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int
     const int it = blockIdx.x * kWarpsPerBlock + warp;
     if (it >= nitems) return;
     ring_fwd_body<RMAX, NB, MIX>(t, o, items[it], jlo, jhi, alm, out, b0, sm[warp], warp, lane);
+}
+
+// the same with the items in blocks, whose warps may share an item's degrees
+template <int RMAX, int NB, bool MIX>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, RMAX >= 4 ? 3 : NB == 1 ? 5 : NB == 2 ? 4 : 3)
+ring_fwd_split_kernel(RingTables t, RingOut o, const RingItem* __restrict__ blocks,
+                      const int* __restrict__ jlo, const int* __restrict__ jhi,
+                      const double2* __restrict__ alm, double2* __restrict__ out, int b0) {
+    __shared__ FwdSmem<NB, MIX> sm[kWarpsPerBlock];
+    __shared__ FwdPart parts[kWarpsPerBlock];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const RingItem item = blocks[blockIdx.x * kWarpsPerBlock + warp];
+    if (item.n == 0) return;
+    ring_fwd_body<RMAX, NB, MIX>(t, o, item, jlo, jhi, alm, out, b0, sm[warp], warp, lane, parts,
+                                 item.pad_ & 0xff, item.pad_ >> 8);
 }
 
 // the forward ring passes of many plans: item i belongs to plan items[i].slot
@@ -1004,9 +1067,16 @@ __global__ void alm_prepare_kernel(double2* __restrict__ alm, int L, int B,
 // launchers
 // ---------------------------------------------------------------------------------------
 template <int RMAX, int NB, bool MIX>
-static int launch_fwd(const RingTables& t, const RingOut& o, const RingItem* items, int nitems,
-                      const int* jlo, const int* jhi, const double2* alm, double2* out, int b0,
-                      cudaStream_t s) {
+static int launch_fwd(const RingTables& t, const RingOut& o, const RingItems& v, const double2* alm,
+                      double2* out, int b0, cudaStream_t s) {
+    const RingItem* items = v.items;
+    const int nitems = v.nitems, *jlo = v.jlo, *jhi = v.jhi;
+    if (v.blocks) {
+        if (v.nblocks <= 0) return 0;
+        ring_fwd_split_kernel<RMAX, NB, MIX><<<v.nblocks, kWarpsPerBlock * 32, 0, s>>>(t, o, v.blocks, jlo, jhi,
+                                                                                       alm, out, b0);
+        return check_launch("ring_fwd_split_kernel");
+    }
     const int grid = (nitems + kWarpsPerBlock - 1) / kWarpsPerBlock;
     ring_fwd_kernel<RMAX, NB, MIX><<<grid, kWarpsPerBlock * 32, 0, s>>>(t, o, items, nitems, jlo, jhi,
                                                                        alm, out, b0);
@@ -1029,14 +1099,14 @@ static int ring_forward_t(const RingTables& t, const RingOut& o, const RingItems
     while (b0 < B) {
         const int rem = B - b0;
         if (rem >= 4) {
-            PF_TRY((launch_fwd<1, 4, MIX>(t, o, it.items, it.nitems, it.jlo, it.jhi, alm, out, b0, s)));
+            PF_TRY((launch_fwd<2, 4, MIX>(t, o, it, alm, out, b0, s)));
             b0 += 4;
         } else if (rem >= 2) {
-            PF_TRY((launch_fwd<2, 2, MIX>(t, o, it.items, it.nitems, it.jlo, it.jhi, alm, out, b0, s)));
+            PF_TRY((launch_fwd<2, 2, MIX>(t, o, it, alm, out, b0, s)));
             b0 += 2;
         } else {
-            if (it.rmax >= 4) PF_TRY((launch_fwd<4, 1, MIX>(t, o, it.items, it.nitems, it.jlo, it.jhi, alm, out, b0, s)));
-            else PF_TRY((launch_fwd<2, 1, MIX>(t, o, it.items, it.nitems, it.jlo, it.jhi, alm, out, b0, s)));
+            if ((it.blocks ? it.block_rmax : it.rmax) >= 4) PF_TRY((launch_fwd<4, 1, MIX>(t, o, it, alm, out, b0, s)));
+            else PF_TRY((launch_fwd<2, 1, MIX>(t, o, it, alm, out, b0, s)));
             b0 += 1;
         }
     }
@@ -1120,6 +1190,77 @@ int build_ring_items(const std::vector<int>& jlo, const std::vector<int>& jhi, i
     return 0;
 }
 
+// blocks of the forward for each group of orders [bounds[k], bounds[k + 1]), the group's blocks at
+// [off[k], off[k + 1]): (order, tile) pairs split into 4, 2 or 1 pieces of degrees, one warp each;
+// pieces of one pair in one block, longest blocks first
+std::vector<RingItem> make_fwd_blocks(const std::vector<int>& jlo, const std::vector<int>& jhi, int L, int mmax,
+                                      int tile, const RingSegments& seg, const std::vector<int>& bounds,
+                                      std::vector<int>& off) {
+    const std::vector<RingItem> pairs = make_ring_items(jlo, jhi, L, mmax, tile);
+    auto pieces = [&](const RingItem& p) {
+        const int K = seg.seg_degrees > 0 ? seg.nseg[p.m] : 1;
+        return K >= 4 ? 4 : K >= 2 ? 2 : 1;
+    };
+    std::vector<RingItem> flat;
+    off.assign(1, 0);
+    for (size_t g = 0; g + 1 < bounds.size(); ++g) {
+        std::vector<RingItem> by[3];  // split into 4, 2, 1
+        for (const RingItem& p : pairs)
+            if (p.m >= bounds[g] && p.m < bounds[g + 1]) by[pieces(p) == 4 ? 0 : pieces(p) == 2 ? 1 : 2].push_back(p);
+        struct Block {
+            int64_t cost;  // of its longest piece
+            RingItem it[kFwdBlockItems];
+        };
+        std::vector<Block> blocks;
+        for (int c = 0; c < 3; ++c) {
+            const int size = c == 0 ? 4 : c == 1 ? 2 : 1, per = kFwdBlockItems / size;
+            for (size_t i = 0; i < by[c].size(); i += per) {
+                Block b;
+                b.cost = (int64_t)((by[c][i].n + 31) / 32) * (L - by[c][i].m + 1) / size;
+                for (int w = 0; w < kFwdBlockItems; ++w) {
+                    const size_t k = i + w / size;
+                    const int q = w % size;
+                    if (k >= by[c].size()) {
+                        b.it[w] = RingItem{0, 0, 0, 0, 0, -1, -1, split_code(1, 0)};
+                        continue;
+                    }
+                    RingItem it = by[c][k];
+                    const int K = seg.seg_degrees > 0 ? seg.nseg[it.m] : 1;
+                    const int s0 = (int)((int64_t)q * K / size), s1 = (int)((int64_t)(q + 1) * K / size);
+                    if (s0 > 0) {
+                        it.flags &= ~kItemFirst;
+                        it.lbeg = seg.seg_first(it.m, s0);
+                        it.ck = (int)(seg.ckbase[it.m] + (int64_t)(s0 - 1) * (jhi[it.m] - jlo[it.m] + 1) +
+                                      (it.j0 - jlo[it.m]));
+                    }
+                    if (s1 < K) it.lend = seg.seg_first(it.m, s1) - 1;
+                    it.pad_ = split_code(size, q);
+                    b.it[w] = it;
+                }
+                blocks.push_back(b);
+            }
+        }
+        std::stable_sort(blocks.begin(), blocks.end(), [](const Block& a, const Block& b) { return a.cost > b.cost; });
+        for (const Block& b : blocks) flat.insert(flat.end(), b.it, b.it + kFwdBlockItems);
+        off.push_back((int)(flat.size() / kFwdBlockItems));
+    }
+    return flat;
+}
+
+int build_fwd_blocks(const std::vector<int>& jlo, const std::vector<int>& jhi, int L, int mmax, int rmax,
+                     const RingSegments& seg, RingItemsOwner& own, cudaStream_t s) {
+    std::vector<int> off;
+    const std::vector<RingItem> flat = make_fwd_blocks(jlo, jhi, L, mmax, 32 * rmax, seg, {0, L + 1}, off);
+    own.view.block_rmax = rmax;
+    PF_TRY(own.blocks.alloc(sizeof(RingItem) * std::max<size_t>(flat.size(), 1)));
+    if (!flat.empty())
+        PF_CUDA(cudaMemcpyAsync(own.blocks.p, flat.data(), sizeof(RingItem) * flat.size(), cudaMemcpyHostToDevice, s));
+    PF_CUDA(cudaStreamSynchronize(s));
+    own.view.blocks = flat.empty() ? nullptr : own.blocks.as<RingItem>();
+    own.view.nblocks = (int)(flat.size() / kFwdBlockItems);
+    return 0;
+}
+
 // ---------------------------------------------------------------------------------------
 // batched ring passes: the items of many plans, grouped by kernel shape
 // ---------------------------------------------------------------------------------------
@@ -1140,7 +1281,8 @@ int alm_prepare_ptr(void* const* ptrs, int ptr, int L, int B, const unsigned cha
     return check_launch("alm_prepare_ptr_kernel");
 }
 
-// the passes a single-plan launch would make over B transforms: (rings per lane, transforms)
+// a batched plan's passes over its B transforms: (rings per lane, transforms). Four transforms run
+// one ring per lane here (two, the single plan's shape, spill in the persistent kernel: 0.5% slower)
 static std::vector<std::pair<int, int>> ring_passes(int B, int rmax, bool adjoint, std::vector<int>& b0s) {
     std::vector<std::pair<int, int>> v;
     b0s.clear();
