@@ -78,6 +78,10 @@ struct pfsht_plan {
     DevBuf gidx, fg, acc;
     pfsht_plan_info info{};
     StageClock clk;
+    // solve!'s workspace where it is small (solve.cu), the pinned copies of its state and their events
+    DevBuf solve_ws;
+    void* solve_host = nullptr;
+    cudaEvent_t solve_ev[2] = {nullptr, nullptr};
     // an asynchronous host adjoint's zeroing of its output's padding rows, on a host thread
     std::future<void> host_zero;
     ~pfsht_plan() {
@@ -94,6 +98,9 @@ struct pfsht_plan {
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : ev_blk) cudaEventDestroy(e);
         for (cudaEvent_t e : clk.ev) cudaEventDestroy(e);
+        for (cudaEvent_t e : solve_ev)
+            if (e) cudaEventDestroy(e);
+        if (solve_host) cudaFreeHost(solve_host);
     }
 };
 

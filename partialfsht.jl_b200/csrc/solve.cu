@@ -1,15 +1,18 @@
 // solve!(alm, plan, f; mode, rtol, maxiter, prior, w) (src/Analysis.jl:375-436) on the device:
 // conjugate gradients on the normal equations (A^H W A + C^-1) alm = A^H W f.
 //
-// The loop stays on the device. One iteration -- forward apply, point weights, adjoint apply,
-// prior, the two dot products and the three vector updates -- is captured once as a CUDA graph;
-// every scalar (alpha, beta, the residual norms, the iteration count) lives in device memory and
-// is computed by the kernels, so a launch needs nothing from the host. Once the relative residual
-// reaches the tolerance a device flag freezes the updates, exactly where the reference's loop
-// breaks. The host keeps one iteration in flight: it launches iteration i, then waits for the
-// state copied out after iteration i - 1, and stops when that says done (the iteration in flight
-// is then a frozen no-op). Dot products reduce in a fixed order (per-block partials, then one
-// block); the adjoint apply inside an iteration adds floating-point atomically (ring tiles of one
+// The loop stays on the device. An iteration is the forward apply, point weights, adjoint apply,
+// prior, the two dot products and the three vector updates (three kernels: the last block of a
+// dot product also makes the scalar that follows from it); every scalar (alpha, beta, the residual
+// norms, the iteration count) lives in device memory and is computed by the kernels, so a launch
+// needs nothing from the host. Once the relative residual reaches the tolerance a device flag
+// freezes the updates, exactly where the reference's loop breaks. The host keeps one iteration in
+// flight: it launches iteration i, then waits for the state copied out after iteration i - 1, and
+// stops when that says done (the iteration in flight is then a frozen no-op). The launches go
+// straight to the caller's stream: an iteration's kernels take longer than their launches (109
+// against about 60 us at lmax 256), while capturing them as a graph for each solve, with the
+// workspace allocated and freed each time, cost 4 ms and more (8 iterations at lmax 384: 5.9 ms
+// against 1.1). Dot products reduce in a fixed order (per-block partials, then one block); the adjoint apply inside an iteration adds floating-point atomically (ring tiles of one
 // order, spread rows shared by neighbouring bins), so two solves agree to round-off, not bit for
 // bit.
 #include <cuda_runtime.h>
@@ -28,10 +31,11 @@ struct SolveState {
     double2 rsold, rsnew, pAp, alpha, beta;
     double rhsn, rel, tol;
     int iters, done;
+    unsigned blocks;  // blocks of the running dot product that have left their partial sum
 };
 
 struct HostState {
-    double rel;
+    double rel, tol;
     int iters, done;
 };
 
@@ -54,9 +58,8 @@ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
 }
 
 // per-block partial sums of conj(x) y
-__global__ void __launch_bounds__(kThreads) dot_partial_kernel(const double2* __restrict__ x,
-                                                               const double2* __restrict__ y,
-                                                               int64_t n, double2* __restrict__ part) {
+__device__ __forceinline__ void dot_partial(const double2* __restrict__ x, const double2* __restrict__ y,
+                                            int64_t n, double2* __restrict__ part) {
     __shared__ double2 sh[kThreads];
     double sr = 0.0, si = 0.0, tr = 0.0, ti = 0.0;
     const int64_t step = (int64_t)gridDim.x * kThreads;
@@ -85,12 +88,27 @@ __global__ void __launch_bounds__(kThreads) dot_partial_kernel(const double2* __
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-__device__ double2 reduce_parts(const double2* __restrict__ part) {
+// whether this block is the last of the grid to have left its partial sum (which it can then read)
+__device__ bool last_block(SolveState* st) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(&st->blocks, 1u) == gridDim.x - 1;
+        if (last) st->blocks = 0;
+    }
+    __syncthreads();
+    __threadfence();
+    return last;
+}
+
+__device__ double2 reduce_parts(const double2* part) {
     __shared__ double2 sh[kThreads];
     double sr = 0.0, si = 0.0;
     for (int k = threadIdx.x; k < kDotBlocks; k += kThreads) {
-        sr += part[k].x;
-        si += part[k].y;
+        const double2 v = __ldcg(part + k);
+        sr += v.x;
+        si += v.y;
     }
     sh[threadIdx.x] = make_double2(sr, si);
     __syncthreads();
@@ -104,9 +122,11 @@ __device__ double2 reduce_parts(const double2* __restrict__ part) {
     return sh[0];
 }
 
-// initial state: rsold = dot(r, r), rhsn = sqrt|dot(rhs, rhs)| (r = rhs)
-__global__ void __launch_bounds__(kThreads) init_state_kernel(const double2* __restrict__ part,
-                                                              SolveState* st, double tol) {
+// initial state: rsold = dot(r, r), rhsn = sqrt|dot(rhs, rhs)| (r = rhs); st->blocks is 0
+__global__ void __launch_bounds__(kThreads) init_state_kernel(const double2* __restrict__ r, int64_t n,
+                                                              double2* part, SolveState* st, double tol) {
+    dot_partial(r, r, n, part);
+    if (!last_block(st)) return;
     const double2 d = reduce_parts(part);
     if (threadIdx.x == 0) {
         st->rsold = d;
@@ -120,7 +140,11 @@ __global__ void __launch_bounds__(kThreads) init_state_kernel(const double2* __r
 }
 
 // alpha = rsold / dot(p, Ap) (0 when the denominator is 0)
-__global__ void __launch_bounds__(kThreads) alpha_kernel(const double2* __restrict__ part, SolveState* st) {
+__global__ void __launch_bounds__(kThreads) alpha_kernel(const double2* __restrict__ p,
+                                                         const double2* __restrict__ Ap, int64_t n,
+                                                         double2* part, SolveState* st) {
+    dot_partial(p, Ap, n, part);
+    if (!last_block(st)) return;
     const double2 d = reduce_parts(part);
     if (threadIdx.x == 0 && !st->done) {
         st->pAp = d;
@@ -128,14 +152,13 @@ __global__ void __launch_bounds__(kThreads) alpha_kernel(const double2* __restri
     }
 }
 
-// alm += alpha p; r -= alpha Ap; and the per-block partial sums of |r|^2 of the new residual
-// (for dot(r, r)) in the same pass. Frozen: r is unchanged and the partials are its norm.
+// alm += alpha p; r -= alpha Ap; and rsnew = dot(r, r) of the new residual in the same pass: count
+// the iteration, stop at rel <= tol, else beta = rsnew / rsold. Frozen: nothing changes.
 __global__ void __launch_bounds__(kThreads) update_xr_kernel(double2* __restrict__ alm,
                                                              double2* __restrict__ r,
                                                              const double2* __restrict__ p,
                                                              const double2* __restrict__ Ap, int64_t n,
-                                                             const SolveState* __restrict__ st,
-                                                             double2* __restrict__ part) {
+                                                             SolveState* st, double2* part) {
     __shared__ double2 sh[kThreads];
     const bool frozen = st->done != 0;
     const double2 a = st->alpha;
@@ -161,10 +184,7 @@ __global__ void __launch_bounds__(kThreads) update_xr_kernel(double2* __restrict
         __syncthreads();
     }
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-// rsnew = dot(r, r); count the iteration; stop at rel <= tol, else beta = rsnew / rsold
-__global__ void __launch_bounds__(kThreads) rsnew_kernel(const double2* __restrict__ part, SolveState* st) {
+    if (!last_block(st)) return;
     const double2 d = reduce_parts(part);
     if (threadIdx.x == 0 && !st->done) {
         st->iters += 1;
@@ -218,9 +238,9 @@ __global__ void prior_kernel(double2* __restrict__ Ap, const double2* __restrict
 
 unsigned grid_n(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, 148 * 16)); }
 
-struct SolveBufs {
-    DevBuf rhs, r, p, Ap, fbuf, fw, part, state, reg;
-};
+// the workspace of one solve: kept with the plan up to this size, so that a program's further solves
+// allocate nothing; a larger one is given back when the solve ends
+constexpr size_t kKeepBytes = (size_t)256 << 20;
 
 int run_solve(pfsht_plan* pl, const double2* f, double2* alm, int mode, double rtol, int maxiter,
               const double* prior, const double* w, cudaStream_t s, int* iters_out, double* rel_out) {
@@ -228,30 +248,38 @@ int run_solve(pfsht_plan* pl, const double2* f, double2* alm, int mode, double r
     const int64_t nc = (int64_t)(L + 1) * (2 * L + 1) * B;
     const int64_t nf = pl->M * B;
     const size_t ca = sizeof(double2) * nc, cf = sizeof(double2) * nf;
-    SolveBufs b;
-    PF_TRY(b.rhs.alloc(ca));
-    PF_TRY(b.r.alloc(ca));
-    PF_TRY(b.p.alloc(ca));
-    PF_TRY(b.Ap.alloc(ca));
-    PF_TRY(b.fbuf.alloc(cf));
-    PF_TRY(b.fw.alloc(cf));
-    PF_TRY(b.part.alloc(sizeof(double2) * kDotBlocks));
-    PF_TRY(b.state.alloc(sizeof(SolveState)));
-    const double2* d_rhs = b.rhs.as<double2>();
-    double2* d_r = b.r.as<double2>();
-    double2* d_p = b.p.as<double2>();
-    double2* d_Ap = b.Ap.as<double2>();
-    double2* d_f = b.fbuf.as<double2>();
-    double2* d_part = b.part.as<double2>();
-    SolveState* st = b.state.as<SolveState>();
+    // r, p, Ap, the field, the partial sums, the state, the prior's inverse
+    size_t at = 0;
+    auto place = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) / 256 * 256;
+        return o;
+    };
+    const size_t o_r = place(ca), o_p = place(ca), o_Ap = place(ca), o_f = place(cf),
+                 o_part = place(sizeof(double2) * kDotBlocks), o_st = place(sizeof(SolveState)),
+                 o_reg = place(sizeof(double) * (L + 1));
+    DevBuf own;
+    DevBuf& ws = at <= kKeepBytes ? pl->solve_ws : own;
+    if (ws.bytes < at) PF_TRY(ws.alloc(at));
+    unsigned char* base = ws.as<unsigned char>();
+    double2* d_r = reinterpret_cast<double2*>(base + o_r);
+    double2* d_p = reinterpret_cast<double2*>(base + o_p);
+    double2* d_Ap = reinterpret_cast<double2*>(base + o_Ap);
+    double2* d_f = reinterpret_cast<double2*>(base + o_f);
+    double2* d_part = reinterpret_cast<double2*>(base + o_part);
+    SolveState* st = reinterpret_cast<SolveState*>(base + o_st);
     const double* d_reg = nullptr;
+    if (!pl->solve_host) PF_CUDA(cudaHostAlloc(&pl->solve_host, 2 * sizeof(HostState), cudaHostAllocDefault));
+    for (cudaEvent_t& e : pl->solve_ev)
+        if (!e) PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    HostState* hs = static_cast<HostState*>(pl->solve_host);
+    std::vector<double> reg;
     if (mode == PFSHT_SOLVE_WIENER) {
         // _prior_inverse! (src/Analysis.jl:437-447): 1 / C_l where C_l > 0, else 0
-        std::vector<double> reg(L + 1);
+        reg.resize(L + 1);
         for (int l = 0; l <= L; ++l) reg[l] = prior[l] > 0 ? 1.0 / prior[l] : 0.0;
-        PF_TRY(b.reg.alloc(sizeof(double) * (L + 1)));
-        PF_CUDA(cudaMemcpyAsync(b.reg.p, reg.data(), sizeof(double) * (L + 1), cudaMemcpyHostToDevice, s));
-        d_reg = b.reg.as<double>();
+        PF_CUDA(cudaMemcpyAsync(base + o_reg, reg.data(), sizeof(double) * (L + 1), cudaMemcpyHostToDevice, s));
+        d_reg = reinterpret_cast<const double*>(base + o_reg);
     }
     const double tol = mode == PFSHT_SOLVE_MINNORM ? std::min(rtol, 1e-12) : rtol;
     // the solve's applies are not stage-timed
@@ -263,19 +291,30 @@ int run_solve(pfsht_plan* pl, const double2* f, double2* alm, int mode, double r
         ~Restore() { p->clk.on = on; }
     } restore{pl, clk_on};
 
-    // rhs = A^H (w f); alm = 0; r = p = rhs
-    PF_CUDA(cudaMemcpyAsync(b.fw.p, f, cf, cudaMemcpyDeviceToDevice, s));
+    // whatever ends the solve, nothing of it is left running on the workspace
+    struct Drain {
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
+    } drain{s};
+    auto copy_state = [&](int k) -> int {
+        PF_CUDA(cudaMemcpyAsync(hs + k, &st->rel, sizeof(HostState), cudaMemcpyDeviceToHost, s));
+        PF_CUDA(cudaEventRecord(pl->solve_ev[k], s));
+        return 0;
+    };
+
+    // r = p = A^H (w f); alm = 0
+    PF_CUDA(cudaMemsetAsync(st, 0, sizeof(SolveState), s));
+    const double2* rhs_field = f;
     if (w) {
-        weight_kernel<<<grid_n(nf), kThreads, 0, s>>>(b.fw.as<double2>(), w, pl->M, B);
+        PF_CUDA(cudaMemcpyAsync(d_f, f, cf, cudaMemcpyDeviceToDevice, s));
+        weight_kernel<<<grid_n(nf), kThreads, 0, s>>>(d_f, w, pl->M, B);
         PF_TRY(check_launch("weight_kernel"));
+        rhs_field = d_f;
     }
-    PF_TRY(pfsht_adjoint(pl, b.fw.p, b.rhs.p, s) == PFSHT_OK ? 0 : PFSHT_ERR_CUDA);
+    PF_TRY(pfsht_adjoint(pl, rhs_field, d_r, s) == PFSHT_OK ? 0 : PFSHT_ERR_CUDA);
     PF_CUDA(cudaMemsetAsync(alm, 0, ca, s));
-    PF_CUDA(cudaMemcpyAsync(d_r, d_rhs, ca, cudaMemcpyDeviceToDevice, s));
-    PF_CUDA(cudaMemcpyAsync(d_p, d_rhs, ca, cudaMemcpyDeviceToDevice, s));
-    dot_partial_kernel<<<kDotBlocks, kThreads, 0, s>>>(d_r, d_r, nc, d_part);
-    PF_TRY(check_launch("dot_partial_kernel"));
-    init_state_kernel<<<1, kThreads, 0, s>>>(d_part, st, tol);
+    PF_CUDA(cudaMemcpyAsync(d_p, d_r, ca, cudaMemcpyDeviceToDevice, s));
+    init_state_kernel<<<kDotBlocks, kThreads, 0, s>>>(d_r, nc, d_part, st, tol);
     PF_TRY(check_launch("init_state_kernel"));
     SolveState h0;
     PF_CUDA(cudaMemcpyAsync(&h0, st, sizeof(h0), cudaMemcpyDeviceToHost, s));
@@ -286,69 +325,27 @@ int run_solve(pfsht_plan* pl, const double2* f, double2* alm, int mode, double r
         return 0;
     }
 
-    // one iteration, captured
-    cudaStream_t cs;
-    PF_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    struct Cleanup {
-        cudaStream_t s;
-        cudaGraph_t* g;
-        cudaGraphExec_t* e;
-        ~Cleanup() {
-            if (*e) cudaGraphExecDestroy(*e);
-            if (*g) cudaGraphDestroy(*g);
-            cudaStreamDestroy(s);
-        }
-    } cleanup{cs, &graph, &exec};
-    PF_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    int rc = pfsht_forward(pl, d_p, d_f, cs) == PFSHT_OK ? 0 : PFSHT_ERR_CUDA;
-    if (!rc && w) {
-        weight_kernel<<<grid_n(nf), kThreads, 0, cs>>>(d_f, w, pl->M, B);
-        rc = check_launch("weight_kernel");
-    }
-    if (!rc) rc = pfsht_adjoint(pl, d_f, d_Ap, cs) == PFSHT_OK ? 0 : PFSHT_ERR_CUDA;
-    if (!rc && d_reg) {
-        prior_kernel<<<grid_n(nc), kThreads, 0, cs>>>(d_Ap, d_p, d_reg, L, B);
-        rc = check_launch("prior_kernel");
-    }
-    if (!rc) {
-        dot_partial_kernel<<<kDotBlocks, kThreads, 0, cs>>>(d_p, d_Ap, nc, d_part);
-        alpha_kernel<<<1, kThreads, 0, cs>>>(d_part, st);
-        update_xr_kernel<<<kDotBlocks, kThreads, 0, cs>>>(alm, d_r, d_p, d_Ap, nc, st, d_part);
-        rsnew_kernel<<<1, kThreads, 0, cs>>>(d_part, st);
-        update_p_kernel<<<grid_n(nc), kThreads, 0, cs>>>(d_p, d_r, nc, st);
-        rc = check_launch("solve iteration kernels");
-    }
-    const cudaError_t ec = cudaStreamEndCapture(cs, &graph);
-    if (rc) return rc;
-    if (ec != cudaSuccess) return fail(PFSHT_ERR_CUDA, cudaGetErrorString(ec));
-    PF_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-
     // one iteration in flight: launch i, then read the state copied out after i - 1
-    HostState* hs = nullptr;
-    PF_CUDA(cudaHostAlloc(&hs, 2 * sizeof(HostState), cudaHostAllocDefault));
-    struct FreeHost {
-        HostState* h;
-        ~FreeHost() { cudaFreeHost(h); }
-    } free_host{hs};
-    cudaEvent_t ev[2];
-    PF_CUDA(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
-    PF_CUDA(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
-    struct FreeEv {
-        cudaEvent_t* e;
-        ~FreeEv() {
-            cudaEventDestroy(e[0]);
-            cudaEventDestroy(e[1]);
-        }
-    } free_ev{ev};
     for (int i = 0; i < maxiter; ++i) {
-        PF_CUDA(cudaGraphLaunch(exec, s));
-        PF_CUDA(cudaMemcpyAsync(&hs[i & 1].rel, &st->rel, sizeof(double), cudaMemcpyDeviceToHost, s));
-        PF_CUDA(cudaMemcpyAsync(&hs[i & 1].iters, &st->iters, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-        PF_CUDA(cudaEventRecord(ev[i & 1], s));
+        PF_TRY(pfsht_forward(pl, d_p, d_f, s) == PFSHT_OK ? 0 : PFSHT_ERR_CUDA);
+        if (w) {
+            weight_kernel<<<grid_n(nf), kThreads, 0, s>>>(d_f, w, pl->M, B);
+            PF_TRY(check_launch("weight_kernel"));
+        }
+        PF_TRY(pfsht_adjoint(pl, d_f, d_Ap, s) == PFSHT_OK ? 0 : PFSHT_ERR_CUDA);
+        if (d_reg) {
+            prior_kernel<<<grid_n(nc), kThreads, 0, s>>>(d_Ap, d_p, d_reg, L, B);
+            PF_TRY(check_launch("prior_kernel"));
+        }
+        alpha_kernel<<<kDotBlocks, kThreads, 0, s>>>(d_p, d_Ap, nc, d_part, st);
+        PF_TRY(check_launch("alpha_kernel"));
+        update_xr_kernel<<<kDotBlocks, kThreads, 0, s>>>(alm, d_r, d_p, d_Ap, nc, st, d_part);
+        PF_TRY(check_launch("update_xr_kernel"));
+        update_p_kernel<<<grid_n(nc), kThreads, 0, s>>>(d_p, d_r, nc, st);
+        PF_TRY(check_launch("update_p_kernel"));
+        PF_TRY(copy_state(i & 1));
         if (i >= 1) {
-            PF_CUDA(cudaEventSynchronize(ev[(i - 1) & 1]));
+            PF_CUDA(cudaEventSynchronize(pl->solve_ev[(i - 1) & 1]));
             if (hs[(i - 1) & 1].done) break;
         }
     }
