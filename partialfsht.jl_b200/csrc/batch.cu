@@ -214,6 +214,8 @@ int batch_create(pfsht_plan* const* plans, int n, int nstreams, pfsht_batch** ou
         pfsht_plan* p = plans[i];
         const size_t nf = sizeof(double2) * (size_t)p->M * p->B;
         if (!p->st_f.p) PF_TRY(p->st_f.alloc(nf));
+        // a Direct plan's own applies need no column array; the merged ring passes do
+        if (!p->H.p) PF_TRY(p->H.alloc(sizeof(double2) * (size_t)p->ro_cols.bstride * p->B));
         stf[i] = p->st_f.as<double2>();
         RingSlot& s = slots[i];
         s.t = p->rt;

@@ -118,6 +118,7 @@ struct RingOut {
     double spin_sgn = 1.0;
     int nrings_out = 0;   // rings of the ring set (rows 0..nrings_out-1 belong to rings)
     int zero_rest = 0;    // forward writes zeros for the rings an order does not retain
+    const double* phi = nullptr;  // adjoint of the Direct leaf: the points' longitudes (ring_data)
 };
 
 // device view of one item list
@@ -227,6 +228,14 @@ int ring_forward(const RingTables& t, const RingOut& o, const RingItems& it, con
 // not store), e.g. on another stream ahead of the pass
 int ring_adjoint(const RingTables& t, const RingOut& o, const RingItems& it, const double2* in,
                  double2* alm, int B, cudaStream_t s, bool prepare = true);
+// Direct synthesis: points per lane, tiles of 32 R points, groups of orders; parts holds
+// groups x B x M values (unused with one group)
+struct DirectShape {
+    int R = 1, tiles = 1, groups = 1;
+};
+DirectShape direct_shape(int64_t M, int lmax, int B);
+int direct_forward(const RingTables& t, const double* phi, int64_t M, const DirectShape& d, const double2* alm,
+                   double2* parts, double2* f, int B, cudaStream_t s);
 int ring_adjoint_prepare(const RingTables& t, const RingItems& it, double2* alm, int B, cudaStream_t s);
 
 // ---------------------------------------------------------------------------------------

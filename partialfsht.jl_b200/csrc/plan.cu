@@ -222,7 +222,7 @@ void fill_info(pfsht_plan* p) {
     int64_t bytes = 0;
     for (const DevBuf* b : {&p->cos_t, &p->log2sin, &p->log2c, &p->w, &p->ab, &p->aboff, &p->fwd_items.items, &p->adj_items.items,
                             &p->adj_seg.ck_p, &p->adj_seg.ck_E, &p->fwd_seg.ck_p, &p->fwd_seg.ck_E, &p->fwd_items.blocks,
-                            &p->H, &p->phi_pts, &p->nd.pts, &p->nd.perm, &p->nd.binstart,
+                            &p->H, &p->direct_parts, &p->phi_pts, &p->nd.pts, &p->nd.perm, &p->nd.binstart,
                             &p->nd.binorder, &p->nd.sorder, &p->nd.bslot, &p->nd.sslot,
                             &p->nd.iorder, &p->nd.items, &p->nd.soff, &p->nd.smeta, &p->nd.ipts, &p->nd.iperm, &p->nd.counter,
                             &p->nd.colp2, &p->nd.p2col, &p->nd.mult1, &p->nd.dec2, &p->nd.pad,
@@ -311,6 +311,12 @@ int build_adjoint_items(pfsht_plan* p, const std::vector<int>& jlo, const std::v
     }
     return build_ring_items(jlo, jhi, L, mmax, rmax, p->adj_items, s,
                             p->adj_seg.seg_degrees > 0 ? &p->adj_seg : nullptr, tile);
+}
+
+// The Direct leaf's FP64 scalar applies take the points' phases inside their ring passes (eight rings
+// per lane, an option, keep the column array)
+bool fused_direct(const pfsht_plan* p) {
+    return p->spin == 0 && p->precision != PFSHT_PRECISION_MIXED && p->R <= 4;
 }
 
 // The forward's blocks: each (order, tile of rings) split into up to four pieces of at least 64
@@ -461,7 +467,6 @@ int build_direct_rings(pfsht_plan* p, const double* h_theta, cudaStream_t s) {
     p->rt.nrings = (int)M;
     p->rt_fwd = p->rt;
     PF_TRY(build_ring_items(jlo, jhi, L, L, p->R > 0 ? p->R : 2, p->fwd_items, s));
-    if (!mix) PF_TRY(build_forward_blocks(p, jlo, jhi, L, s));
     return build_adjoint_items(p, jlo, jhi, L, s);
 }
 
@@ -482,7 +487,13 @@ int build_direct(pfsht_plan* p, const double* h_theta, const double* h_phi, cuda
     p->ro_cols.spin_sgn = 1.0;
     p->ro_cols.nrings_out = (int)M;
     p->ro_cols.zero_rest = 0;  // every point keeps every order
-    PF_TRY(p->H.alloc(sizeof(double2) * (size_t)M * (2 * L + 1) * B));
+    if (fused_direct(p)) {
+        // no column array (a batch, whose merged ring passes write one, allocates it)
+        p->direct = direct_shape(M, L, B);
+        if (p->direct.groups > 1) PF_TRY(p->direct_parts.alloc(sizeof(double2) * (size_t)M * B * p->direct.groups));
+    } else {
+        PF_TRY(p->H.alloc(sizeof(double2) * (size_t)M * (2 * L + 1) * B));
+    }
     return 0;
 }
 
@@ -791,6 +802,12 @@ int plan_create(const double* theta, const double* phi, int64_t npts, int lmax, 
 int apply_forward(pfsht_plan* p, const double2* alm, double2* f, cudaStream_t s) {
     if (p->kind == kMultiBox) return multibox_forward(p, alm, f, s);
     clock_begin(&p->clk, s);
+    if (p->kind == kDirect && fused_direct(p)) {
+        PF_TRY(direct_forward(p->rt_fwd, p->phi_pts.as<double>(), p->M, p->direct, alm, p->direct_parts.as<double2>(),
+                              f, p->B, s));
+        clock_mark(&p->clk, kStDirect, s);
+        return 0;
+    }
     if (p->spin != 0)
         PF_TRY(spin_ring_forward(p->spt.t, p->ro_cols, p->fwd_items.view, alm, p->H.as<double2>(), p->B, s));
     else
@@ -801,6 +818,15 @@ int apply_forward(pfsht_plan* p, const double2* alm, double2* f, cudaStream_t s)
 
 int apply_adjoint(pfsht_plan* p, const double2* f, double2* alm, cudaStream_t s) {
     if (p->kind == kMultiBox) return multibox_adjoint(p, f, alm, s);
+    if (p->kind == kDirect && fused_direct(p)) {
+        clock_begin(&p->clk, s);
+        RingOut o = p->ro_cols;
+        o.phi = p->phi_pts.as<double>();
+        o.bstride = p->M;
+        PF_TRY(ring_adjoint(p->rt, o, p->adj_items.view, f, alm, p->B, s));
+        clock_mark(&p->clk, kStDirect, s);
+        return 0;
+    }
     // zero what the ring pass will not store on the side stream, overlapped with the NUFFT and
     // Theta-FFT stages (a bandwidth-bound fill beside compute-bound kernels); joined before the pass
     PF_CUDA(cudaEventRecord(p->ev_fork, s));

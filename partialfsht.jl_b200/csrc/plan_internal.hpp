@@ -49,7 +49,8 @@ struct pfsht_plan {
     NufftGrid ng;
     NufftDev nd;
     // direct leaf
-    DevBuf phi_pts;
+    DevBuf phi_pts, direct_parts;
+    DirectShape direct;
     // host-buffer staging: st_alm / st_f serve the forward (coefficients in, field out),
     // st_alm2 / st_f2 the adjoint (field in, coefficients out), so that a forward's output copy
     // and an adjoint's input copy (or the next call's) can be in flight while the other computes

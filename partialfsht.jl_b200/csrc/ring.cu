@@ -340,12 +340,12 @@ struct FwdPart {
     double2 p[4][32], m[4][32];
 };
 
+// the sums over an item's degrees: accp / accm times 2^E are the rings' columns of +m and -m
 template <int R, int NB, bool MIX>
-__device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut& o,
-                                              const RingItem& item, const double2* __restrict__ alm,
-                                              double2* __restrict__ out, int b0,
-                                              FwdSmem<NB, MIX>& sm, int warp, int lane,
-                                              FwdPart* parts, int size, int place) {
+__device__ __forceinline__ void ring_fwd_walk(const RingTables& t, const RingItem& item,
+                                              const double2* __restrict__ alm, int b0,
+                                              FwdSmem<NB, MIX>& sm, int lane, int (&E)[R],
+                                              FwdAcc<MIX> (&accp)[R][NB], FwdAcc<MIX> (&accm)[R][NB]) {
     constexpr int STRIDE = MIX ? 16 : 64;
     const int m = item.m, L = t.lmax;
     const double sgn = (m & 1) ? -1.0 : 1.0;
@@ -356,8 +356,6 @@ __device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut
     const double2 zero2 = make_double2(0.0, 0.0);
 
     double x[R], q1[R], q2[R];
-    int E[R];
-    FwdAcc<MIX> accp[R][NB], accm[R][NB];
     const bool seeded = item.ck < 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -534,8 +532,20 @@ __device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut
             fold_all();
         }
     }
+}
+
+template <int R, int NB, bool MIX>
+__device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut& o,
+                                              const RingItem& item, const double2* __restrict__ alm,
+                                              double2* __restrict__ out, int b0,
+                                              FwdSmem<NB, MIX>& sm, int warp, int lane,
+                                              FwdPart* parts, int size, int place) {
+    const int m = item.m;
+    int E[R];
+    FwdAcc<MIX> accp[R][NB], accm[R][NB];
+    ring_fwd_walk<R, NB, MIX>(t, item, alm, b0, sm, lane, E, accp, accm);
     // write the ring columns (window and 2^E folded into one exact scale)
-    const double smir = o.spin_sgn * sgn;
+    const double smir = (m & 1) ? -o.spin_sgn : o.spin_sgn;
     auto write = [&](int k, int b, double2 gp, double2 gm) {
         double2* ob = out + o.bstride * (b0 + b);
         const int j = item.j0 + k;
@@ -671,6 +681,128 @@ ring_fwd_split_kernel(RingTables t, RingOut o, const RingItem* __restrict__ bloc
                                  item.pad_ & 0xff, item.pad_ >> 8);
 }
 
+// ---------------------------------------------------------------------------------------
+// Direct synthesis (src/Direct.jl:60-84): a warp per (tile of 32 R points, group of orders) walks
+// each order m = group, group + groups, ... over its points and adds the columns of +m and -m times
+// e^{+-i m phi} to the points' sums in registers, so no column array is written and read back
+// (49,152 points at lmax 191: 300 MB each way, and 125 us in a kernel of one thread per point that
+// summed the orders one after the other, and took 44 us for 400 points at lmax 64).
+// The groups' sums are added in a fixed order by direct_parts_kernel.
+// ---------------------------------------------------------------------------------------
+constexpr int kDirectWarps = 4;
+template <int R, int NB>
+__global__ void __launch_bounds__(kDirectWarps * 32, R * NB >= 8 ? 2 : R >= 4 ? 3 : 4)
+direct_fwd_kernel(RingTables t, const double* __restrict__ phi, int M, int tiles, int groups,
+                  const double2* __restrict__ alm, int b0, int B, double2* __restrict__ parts) {
+    __shared__ FwdSmem<NB, false> sm[kDirectWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = blockIdx.x * kDirectWarps + warp;
+    if (w >= tiles * groups) return;
+    const int tile = w % tiles, group = w / tiles;
+    const int j0 = tile * 32 * R, n = min(32 * R, M - j0);
+    double ph[R];
+    double2 f[R][NB];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int k = lane + 32 * r;
+        ph[r] = k < n ? phi[j0 + k] : 0.0;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) f[r][b] = make_double2(0.0, 0.0);
+    }
+    for (int m = group; m <= t.lmax; m += groups) {
+        int E[R];
+        FwdAcc<false> accp[R][NB], accm[R][NB];
+        ring_fwd_walk<R, NB, false>(t, whole_item(m, j0, n, 0, t.lmax), alm, b0, sm[warp], lane, E, accp, accm);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            double sn = 0.0, cs = 1.0;
+            if (m > 0) sincos((double)m * ph[r], &sn, &cs);
+            const double sc = scalbn(1.0, E[r]);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const double2 p = accp[r][b].a, q = accm[r][b].a;
+                const double2 gp = make_double2(p.x * sc, p.y * sc), gm = make_double2(q.x * sc, q.y * sc);
+                if (m == 0) {
+                    f[r][b].x += gp.x;
+                    f[r][b].y += gp.y;
+                } else {
+                    f[r][b].x += (gp.x * cs - gp.y * sn) + (gm.x * cs + gm.y * sn);
+                    f[r][b].y += (gp.x * sn + gp.y * cs) + (gm.y * cs - gm.x * sn);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int k = lane + 32 * r;
+        if (k >= n) continue;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) parts[((int64_t)group * B + b0 + b) * M + j0 + k] = f[r][b];
+    }
+}
+
+// f = the sum of the groups' parts, in order
+__global__ void direct_parts_kernel(const double2* __restrict__ parts, int64_t n, int groups,
+                                    double2* __restrict__ f) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double2 s = parts[i];
+#pragma unroll 8
+    for (int g = 1; g < groups; ++g) {
+        const double2 v = parts[g * n + i];
+        s.x += v.x;
+        s.y += v.y;
+    }
+    f[i] = s;
+}
+
+// tiles and order groups for M points: points per lane down to one while the (tile, order) pairs are
+// fewer than the warps of a wave, then groups for about three waves of equal warps
+DirectShape direct_shape(int64_t M, int L, int B) {
+    DirectShape d;
+    const int64_t wave = 148 * 16;
+    auto tiles = [&](int r) { return (M + 32 * r - 1) / (32 * r); };
+    d.R = B > 1 ? 2 : 4;
+    while (d.R > 1 && tiles(d.R) * (L + 1) < wave) d.R /= 2;
+    d.tiles = (int)tiles(d.R);
+    d.groups = (int)std::max<int64_t>(1, std::min<int64_t>(L + 1, (3 * wave + d.tiles - 1) / d.tiles));
+    return d;
+}
+
+template <int R, int NB>
+static int launch_direct(const RingTables& t, const double* phi, int64_t M, const DirectShape& d, const double2* alm,
+                         int b0, int B, double2* parts, cudaStream_t s) {
+    const int64_t warps = (int64_t)d.tiles * d.groups;
+    direct_fwd_kernel<R, NB><<<(unsigned)((warps + kDirectWarps - 1) / kDirectWarps), kDirectWarps * 32, 0, s>>>(
+        t, phi, (int)M, d.tiles, d.groups, alm, b0, B, parts);
+    return check_launch("direct_fwd_kernel");
+}
+
+int direct_forward(const RingTables& t, const double* phi, int64_t M, const DirectShape& d, const double2* alm,
+                   double2* parts, double2* f, int B, cudaStream_t s) {
+    for (int b0 = 0; b0 < B;) {
+        const int rem = B - b0;
+        double2* out = d.groups == 1 ? f : parts;
+        if (rem >= 4) {
+            PF_TRY(d.R >= 2 ? (launch_direct<2, 4>(t, phi, M, d, alm, b0, B, out, s))
+                            : (launch_direct<1, 4>(t, phi, M, d, alm, b0, B, out, s)));
+            b0 += 4;
+        } else if (rem >= 2) {
+            PF_TRY(d.R >= 2 ? (launch_direct<2, 2>(t, phi, M, d, alm, b0, B, out, s))
+                            : (launch_direct<1, 2>(t, phi, M, d, alm, b0, B, out, s)));
+            b0 += 2;
+        } else {
+            PF_TRY(d.R >= 4   ? (launch_direct<4, 1>(t, phi, M, d, alm, b0, B, out, s))
+                   : d.R >= 2 ? (launch_direct<2, 1>(t, phi, M, d, alm, b0, B, out, s))
+                              : (launch_direct<1, 1>(t, phi, M, d, alm, b0, B, out, s)));
+            b0 += 1;
+        }
+    }
+    if (d.groups == 1) return 0;
+    direct_parts_kernel<<<(unsigned)((M * B + 127) / 128), 128, 0, s>>>(parts, M * B, d.groups, f);
+    return check_launch("direct_parts_kernel");
+}
+
 // the forward ring passes of many plans: item i belongs to plan items[i].slot
 template <int RMAX, int NB, bool MIX>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
@@ -701,7 +833,41 @@ struct AdjSmem {  // one warp's staging (a block holds one per warp)
     double2 bg[32];
 };
 
-template <int R, int NB, bool MIX>
+// where the adjoint's ring data come from: the column array, or (phi given) the Direct leaf's values
+// v at the points, whose columns of +m and -m are v e^{-i m phi} and v e^{i m phi}
+// (src/Direct.jl:102-114)
+template <bool PHASE>
+__device__ __forceinline__ void ring_data(const RingOut& o, const double2* __restrict__ ib, int m, int j,
+                                          double smir, double2& vp, double2& vm) {
+    vm = make_double2(0.0, 0.0);
+    if constexpr (PHASE) {
+        const double2 v = ib[j];
+        vp = v;
+        if (m > 0) {
+            double sn, cs;
+            sincos((double)m * o.phi[j], &sn, &cs);
+            vp = make_double2(v.x * cs + v.y * sn, v.y * cs - v.x * sn);
+            vm = make_double2(v.x * cs - v.y * sn, v.y * cs + v.x * sn);
+        }
+    } else {
+        vp = ib[j + o.ld * (o.col_off + m)];
+        if (o.reflect) {
+            const double2 u = ib[(o.nrows - 1 - j) + o.ld * (o.col_off + m)];
+            vp.x += smir * u.x;
+            vp.y += smir * u.y;
+        }
+        if (m > 0) {
+            vm = ib[j + o.ld * (o.col_off - m)];
+            if (o.reflect) {
+                const double2 q = ib[(o.nrows - 1 - j) + o.ld * (o.col_off - m)];
+                vm.x += smir * q.x;
+                vm.y += smir * q.y;
+            }
+        }
+    }
+}
+
+template <int R, int NB, bool MIX, bool PHASE = false>
 __device__ __forceinline__ void ring_adj_item(const RingTables& t, const RingOut& o,
                                               const RingItem& item, const double2* __restrict__ in,
                                               double* __restrict__ almd, int b0, int wmode,
@@ -744,23 +910,10 @@ __device__ __forceinline__ void ring_adj_item(const RingTables& t, const RingOut
         const double sc = scalbn(t.w ? t.w[j] : 1.0, E[r]);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-            const double2* ib = in + o.bstride * (b0 + b);
-            double2 v = ib[j + o.ld * (o.col_off + m)];
-            if (o.reflect) {
-                const double2 u = ib[(o.nrows - 1 - j) + o.ld * (o.col_off + m)];
-                v.x += smir * u.x;
-                v.y += smir * u.y;
-            }
+            double2 v, u;
+            ring_data<PHASE>(o, in + o.bstride * (b0 + b), m, j, smir, v, u);
             gp[r][b] = put(v.x * sc, v.y * sc);
-            if (m > 0) {
-                double2 u = ib[j + o.ld * (o.col_off - m)];
-                if (o.reflect) {
-                    const double2 q = ib[(o.nrows - 1 - j) + o.ld * (o.col_off - m)];
-                    u.x += smir * q.x;
-                    u.y += smir * q.y;
-                }
-                gm[r][b] = put(u.x * sc * sgn, u.y * sc * sgn);
-            }
+            gm[r][b] = put(u.x * sc * sgn, u.y * sc * sgn);
         }
     };
     const bool seeded = item.ck < 0;
@@ -785,23 +938,7 @@ __device__ __forceinline__ void ring_adj_item(const RingTables& t, const RingOut
             if (t.w) wr[r] = t.w[j];
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
-                const double2* ib = in + o.bstride * (b0 + b);
-                double2 v = ib[j + o.ld * (o.col_off + m)];
-                if (o.reflect) {
-                    const double2 u = ib[(o.nrows - 1 - j) + o.ld * (o.col_off + m)];
-                    v.x += smir * u.x;
-                    v.y += smir * u.y;
-                }
-                rp[r][b] = v;
-                if (m > 0) {
-                    double2 u = ib[j + o.ld * (o.col_off - m)];
-                    if (o.reflect) {
-                        const double2 q = ib[(o.nrows - 1 - j) + o.ld * (o.col_off - m)];
-                        u.x += smir * q.x;
-                        u.y += smir * q.y;
-                    }
-                    rm[r][b] = u;
-                }
+                ring_data<PHASE>(o, in + o.bstride * (b0 + b), m, j, smir, rp[r][b], rm[r][b]);
             }
         }
     }
@@ -1000,7 +1137,7 @@ __device__ __forceinline__ void ring_adj_item(const RingTables& t, const RingOut
     }
 }
 
-template <int RMAX, int NB, bool MIX>
+template <int RMAX, int NB, bool MIX, bool PHASE = false>
 __device__ __forceinline__ void ring_adj_body(const RingTables& t, const RingOut& o,
                                               const RingItem& item, const double2* __restrict__ in,
                                               double* __restrict__ almd, int b0, int allow_sole,
@@ -1016,14 +1153,14 @@ __device__ __forceinline__ void ring_adj_body(const RingTables& t, const RingOut
         sub.n = min(32 * RMAX, item.n - base);
         if (sub.ck >= 0) sub.ck += base;
         const int reff = (sub.n + 31) >> 5;
-        if (RMAX >= 8 && reff >= 5) ring_adj_item<(RMAX >= 8 ? 8 : 1), NB, MIX>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
-        else if (RMAX >= 4 && reff >= 3) ring_adj_item<(RMAX >= 4 ? 4 : 1), NB, MIX>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
-        else if (RMAX >= 2 && reff == 2) ring_adj_item<(RMAX >= 2 ? 2 : 1), NB, MIX>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
-        else ring_adj_item<1, NB, MIX>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
+        if (RMAX >= 8 && reff >= 5) ring_adj_item<(RMAX >= 8 ? 8 : 1), NB, MIX, PHASE>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
+        else if (RMAX >= 4 && reff >= 3) ring_adj_item<(RMAX >= 4 ? 4 : 1), NB, MIX, PHASE>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
+        else if (RMAX >= 2 && reff == 2) ring_adj_item<(RMAX >= 2 ? 2 : 1), NB, MIX, PHASE>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
+        else ring_adj_item<1, NB, MIX, PHASE>(t, o, sub, in, almd, b0, wmode, sm, warp, lane);
     }
 }
 
-template <int RMAX, int NB, bool MIX>
+template <int RMAX, int NB, bool MIX, bool PHASE>
 __global__ void __launch_bounds__(kAdjWarps * 32)
 ring_adj_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int nitems,
                 const double2* __restrict__ in, double* __restrict__ almd, int b0, int allow_sole) {
@@ -1031,7 +1168,7 @@ ring_adj_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int it = blockIdx.x * kAdjWarps + warp;
     if (it >= nitems) return;
-    ring_adj_body<RMAX, NB, MIX>(t, o, items[it], in, almd, b0, allow_sole, sm[warp], warp, lane);
+    ring_adj_body<RMAX, NB, MIX, PHASE>(t, o, items[it], in, almd, b0, allow_sole, sm[warp], warp, lane);
 }
 
 // the adjoint ring passes of many plans: item i belongs to plan items[i].slot
@@ -1087,8 +1224,15 @@ template <int RMAX, int NB, bool MIX>
 static int launch_adj(const RingTables& t, const RingOut& o, const RingItem* items, int nitems,
                       const double2* in, double2* alm, int b0, int allow_sole, cudaStream_t s) {
     const int grid = (nitems + kAdjWarps - 1) / kAdjWarps;
-    ring_adj_kernel<RMAX, NB, MIX><<<grid, kAdjWarps * 32, 0, s>>>(
-        t, o, items, nitems, in, reinterpret_cast<double*>(alm), b0, allow_sole);
+    double* out = reinterpret_cast<double*>(alm);
+    if constexpr (!MIX && RMAX <= 4) {
+        if (o.phi) {
+            ring_adj_kernel<RMAX, NB, MIX, true><<<grid, kAdjWarps * 32, 0, s>>>(t, o, items, nitems, in, out, b0,
+                                                                                 allow_sole);
+            return check_launch("ring_adj_kernel");
+        }
+    }
+    ring_adj_kernel<RMAX, NB, MIX, false><<<grid, kAdjWarps * 32, 0, s>>>(t, o, items, nitems, in, out, b0, allow_sole);
     return check_launch("ring_adj_kernel");
 }
 
