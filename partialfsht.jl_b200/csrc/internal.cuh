@@ -332,6 +332,7 @@ struct NufftGrid {
     // of 8 slots; nitems work items of at most item_rows origin rows
     int mma = 0, mma_interp = 0;
     int blk_cols = 1, item_rows = 1 << 20, nitems = 0;
+    int cols = 0;              // the column stages run as one kernel each way (nufft_cols.cu)
     int interp_pipe = 1;       // one-transform interpolation copies the next group's tile ahead
 };
 
@@ -353,7 +354,8 @@ struct NufftDev {
     DevBuf p2col;     // int32 nf2: mode column of each fine column or -1
     DevBuf mult1;     // double2 n1: per-mode complex factor along dim 1 (deconv incl.)
     DevBuf dec2;      // double ncols: deconvolution along dim 2
-    DevBuf pad;       // double2 nf1 x ncols x B
+    DevBuf roots_th, roots_f1;  // double2: roots of unity of the column FFTs (cols)
+    DevBuf pad;       // double2 nf1 x ncols x B (not with cols)
     DevBuf U;         // double2 nrows x nf2 x B
     DevBuf counter;   // int: the next interpolation group to pull
     cufftHandle f1 = 0, f2 = 0;
@@ -382,6 +384,21 @@ int mma_fill_slots(const NufftGrid& g, NufftDev& d, const double2* gg, const int
                    const MmaGroup* groups, int64_t nslots, cudaStream_t s);
 int interp_mma(const NufftGrid& g, NufftDev& d, double2* f, int B, cudaStream_t s);
 int spread_mma(const NufftGrid& g, NufftDev& d, const double2* f, int B, cudaStream_t s);
+
+// The column stages in one kernel each way (nufft_cols.cu), for the leaf's mode columns H before
+// (after) their FFT along Theta: setup_cols decides (g.cols), up to kColsMostCells padded cells of a
+// transform. A forward and adjoint with the library chain against this, us: 0.11 million cells 110
+// against 88, 0.3 125 / 109, 0.6 179 / 155 (four transforms 526 / 494), 0.9 241 / 234 (740 / 732),
+// 1.0 328 / 334, 1.5 386 / 382 (two transforms 690 / 707), 2.65 771 / 792
+constexpr int64_t kColsMostCells = 950000;
+int setup_cols(NufftGrid& g, NufftDev& d, int B, cudaStream_t s);
+int cols_forward(const NufftGrid& g, NufftDev& d, const double2* H, int B, int iflag, cudaStream_t s);
+int cols_adjoint(const NufftGrid& g, NufftDev& d, double2* H, int B, int iflag, cudaStream_t s);
+// type 2 / type 1 of such a grid: H -> f, f -> H
+int nufft_type2_cols(const NufftGrid& g, NufftDev& d, const double2* H, double2* f, int B, int iflag,
+                     cudaStream_t s, StageClock* clk = nullptr);
+int nufft_type1_cols(const NufftGrid& g, NufftDev& d, const double2* f, double2* H, int B, int iflag,
+                     cudaStream_t s, StageClock* clk = nullptr);
 
 // transform points (x = stretched colatitude, y = longitude; both radians) into grid
 // coordinates, sort them into bins, fill pts/perm/binstart. x,y are device arrays.

@@ -606,18 +606,20 @@ int fine_fft_length(int nmin, int64_t batch, bool fp32, cudaStream_t s, int* out
 int nufft_alloc(NufftGrid& g, NufftDev& d, int B) {
     const size_t el = g.fp32 ? sizeof(float2) : sizeof(double2);
     const cufftType ty = g.fp32 ? CUFFT_C2C : CUFFT_Z2Z;
-    PF_TRY(d.pad.alloc(el * (size_t)g.nf1 * g.ncols * B));
+    if (!g.cols) PF_TRY(d.pad.alloc(el * (size_t)g.nf1 * g.ncols * B));
     PF_TRY(d.U.alloc(el * (size_t)g.nrows * g.nf2 * B));
     PF_TRY(d.counter.alloc(sizeof(int)));
-    int n1[1] = {g.nf1};
-    PF_CUFFT(cufftPlanMany(&d.f1, 1, n1, n1, 1, g.nf1, n1, 1, g.nf1, ty, g.ncols * B));
-    d.have_f1 = true;
+    if (!g.cols) {
+        int n1[1] = {g.nf1};
+        PF_CUFFT(cufftPlanMany(&d.f1, 1, n1, n1, 1, g.nf1, n1, 1, g.nf1, ty, g.ncols * B));
+        d.have_f1 = true;
+    }
     int n2[1] = {g.nf2};
     PF_CUFFT(cufftPlanMany(&d.f2, 1, n2, n2, 1, g.nf2, n2, 1, g.nf2, ty, g.nrows * B));
     d.have_f2 = true;
     // tensor maps for the TMA row transposes (the plain kernels serve when the driver has no
     // encoder or the layout does not fit one)
-    d.have_maps = g.gap_ok && !g.plain_transpose &&
+    d.have_maps = !g.cols && g.gap_ok && !g.plain_transpose &&
                   make_tile_map(&d.pad_map, d.pad.p, (int)el, g.nf1, (int64_t)g.ncols * B, 128 / (int)el, 32) == 0 &&
                   make_tile_map(&d.U_map, d.U.p, (int)el, g.nf2, (int64_t)g.nrows * B, 128 / (int)el, 32) == 0;
     return 0;
@@ -1859,6 +1861,31 @@ static int type1_impl(const NufftGrid& g, NufftDev& d, const double2* f, double2
         PF_TRY(check_launch("unpad_kernel"));
     }
     clock_mark(clk, kStUnpad, s);
+    return 0;
+}
+
+int nufft_type2_cols(const NufftGrid& g, NufftDev& d, const double2* H, double2* f, int B, int iflag,
+                     cudaStream_t s, StageClock* clk) {
+    PF_TRY(cols_forward(g, d, H, B, iflag, s));
+    clock_mark(clk, kStRowsFwd, s);
+    PF_CUFFT(cufftSetStream(d.f2, s));
+    PF_TRY(fine_fft(d.f2, d.U.p, false, iflag > 0 ? CUFFT_INVERSE : CUFFT_FORWARD));
+    clock_mark(clk, kStFft2Fwd, s);
+    PF_TRY(interp_any<double>(g, d, f, B, s));
+    clock_mark(clk, kStInterp, s);
+    return 0;
+}
+
+int nufft_type1_cols(const NufftGrid& g, NufftDev& d, const double2* f, double2* H, int B, int iflag,
+                     cudaStream_t s, StageClock* clk) {
+    PF_CUDA(cudaMemsetAsync(d.U.p, 0, sizeof(double2) * (size_t)g.nrows * g.nf2 * B, s));
+    PF_TRY(spread_any<double>(g, d, f, B, s));
+    clock_mark(clk, kStSpread, s);
+    PF_CUFFT(cufftSetStream(d.f2, s));
+    PF_TRY(fine_fft(d.f2, d.U.p, false, iflag > 0 ? CUFFT_INVERSE : CUFFT_FORWARD));
+    clock_mark(clk, kStFft2Adj, s);
+    PF_TRY(cols_adjoint(g, d, H, B, iflag, s));
+    clock_mark(clk, kStRowsAdj, s);
     return 0;
 }
 

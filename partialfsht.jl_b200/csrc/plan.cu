@@ -225,7 +225,7 @@ void fill_info(pfsht_plan* p) {
                             &p->H, &p->direct_parts, &p->phi_pts, &p->nd.pts, &p->nd.perm, &p->nd.binstart,
                             &p->nd.binorder, &p->nd.sorder, &p->nd.bslot, &p->nd.sslot,
                             &p->nd.iorder, &p->nd.items, &p->nd.soff, &p->nd.smeta, &p->nd.ipts, &p->nd.iperm, &p->nd.counter,
-                            &p->nd.colp2, &p->nd.p2col, &p->nd.mult1, &p->nd.dec2, &p->nd.pad,
+                            &p->nd.roots_th, &p->nd.roots_f1, &p->nd.colp2, &p->nd.p2col, &p->nd.mult1, &p->nd.dec2, &p->nd.pad,
                             &p->nd.U, &p->st_alm, &p->st_f, &p->ab_fwd, &p->st_alm2,
                             &p->st_f2, &p->blk_fwd_items, &p->blk_adj_items})
         bytes += (int64_t)b->bytes;
@@ -393,9 +393,6 @@ int build_stretch(pfsht_plan* p, const double* d_theta, const double* d_phi, con
     p->ro_cols.nrings_out = lf.nth_half;
     p->ro_cols.zero_rest = 1;
     PF_TRY(p->H.alloc(sizeof(double2) * (size_t)lf.nth * p->ncols * B));
-    int n[1] = {lf.nth};
-    PF_CUFFT(cufftPlanMany(&p->fth, 1, n, n, 1, lf.nth, n, 1, lf.nth, CUFFT_Z2Z, p->ncols * B));
-    p->have_fth = true;
 
     // points: stretched colatitude and longitude on the device (src/Stretch.jl:202-213)
     DevBuf Th, ph;
@@ -423,6 +420,12 @@ int build_stretch(pfsht_plan* p, const double* d_theta, const double* d_phi, con
                             p->precision == PFSHT_PRECISION_MIXED, o.nufft_fft_lengths, o.nufft_nf1,
                             o.nufft_nf2, s));
     PF_TRY(nufft_setpts(p->ng, p->nd, Th.as<double>(), ph.as<double>(), s));
+    PF_TRY(setup_cols(p->ng, p->nd, B, s));
+    if (!p->ng.cols) {
+        int n[1] = {lf.nth};
+        PF_CUFFT(cufftPlanMany(&p->fth, 1, n, n, 1, lf.nth, n, 1, lf.nth, CUFFT_Z2Z, p->ncols * B));
+        p->have_fth = true;
+    }
     PF_TRY(nufft_alloc(p->ng, p->nd, B));
     return 0;
 }
@@ -861,6 +864,7 @@ int plan_forward_after_ring(pfsht_plan* p, double2* f, cudaStream_t s) {
         clock_mark(clk, kStDirect, s);
         return 0;
     }
+    if (p->ng.cols) return nufft_type2_cols(p->ng, p->nd, p->H.as<double2>(), f, p->B, +1, s, clk);
     PF_CUFFT(cufftSetStream(p->fth, s));
     PF_CUFFT(cufftExecZ2Z(p->fth, p->H.as<cufftDoubleComplex>(), p->H.as<cufftDoubleComplex>(),
                           CUFFT_FORWARD));
@@ -872,6 +876,7 @@ int plan_adjoint_before_ring(pfsht_plan* p, const double2* f, cudaStream_t s) {
     StageClock* clk = &p->clk;
     if (p->kind == kDirect)
         return direct_phase_spread(f, p->phi_pts.as<double>(), p->M, p->L, p->B, p->H.as<double2>(), s);
+    if (p->ng.cols) return nufft_type1_cols(p->ng, p->nd, f, p->H.as<double2>(), p->B, -1, s, clk);
     PF_TRY(nufft_type1(p->ng, p->nd, f, p->H.as<double2>(), p->B, -1, s, clk));
     PF_CUFFT(cufftSetStream(p->fth, s));
     PF_CUFFT(cufftExecZ2Z(p->fth, p->H.as<cufftDoubleComplex>(), p->H.as<cufftDoubleComplex>(),
