@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : 4)
 interp_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
               const int* __restrict__ binstart, const int* __restrict__ iorder, int nbc, int G,
               int nsbc, int BR, int BC, int64_t M, const cx<T>* __restrict__ U, int nrows,
-              int nf2, int row_wrap, int B, double2* __restrict__ f) {
+              int nf2, int row_wrap, double2* __restrict__ f) {
     extern __shared__ __align__(16) unsigned char interp_smem[];
     cx<T>* tile = reinterpret_cast<cx<T>*>(interp_smem);
     // a group of G consecutive bins of one bin row: their points are contiguous in bin order
@@ -968,7 +968,8 @@ interp_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
     // tile rows an odd number of elements apart: a tap's bank class then depends on its row as
     // well as its column, which evens out the classes the points are dealt over
     const int TS = tg.TC | 1;
-    for (int b = 0; b < B; ++b) {
+    {
+        const int b = blockIdx.y;  // transform
         const cx<T>* ub = U + (int64_t)nrows * nf2 * b;
         if (tg.TC <= 32) {
             if (ln < tg.TC) {
@@ -1135,7 +1136,7 @@ template <int W, class T>
 __global__ void __launch_bounds__(SpreadWarps<W>::N * 32)
 spread_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
               const int* __restrict__ binstart, const int* __restrict__ binorder, int nbusy,
-              int nbc, int BR, int BC, int64_t M, const double2* __restrict__ fin, int b,
+              int nbc, int BR, int BC, int64_t M, const double2* __restrict__ fin,
               int nrows, int nf2, int row_wrap, int plain, cx<T>* __restrict__ U) {
     constexpr int KP = SpreadStage<W, T>::KP;
     constexpr int NW = SpreadWarps<W>::N;
@@ -1147,6 +1148,7 @@ spread_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
     const int s = binstart[bin], e = binstart[bin + 1];
     const TileGeom tg = tile_geom<W>(bin, nbc, BR, BC);
     SpreadStage<W, T>& st = stg[warp];
+    const int b = blockIdx.y;  // transform
     cx<T>* ub = U + (int64_t)nrows * nf2 * b;
     const bool col_ok = lane < tg.TC;
     const int gcol = wrap(tg.tc0 + lane, nf2);
@@ -1281,7 +1283,7 @@ template <int W, class T>
 __global__ void __launch_bounds__(128)
 spread16_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
                 const int* __restrict__ binstart, const int* __restrict__ binorder, int nbusy,
-                int nbc, int BR, int BC, int64_t M, const double2* __restrict__ fin, int b,
+                int nbc, int BR, int BC, int64_t M, const double2* __restrict__ fin,
                 int nrows, int nf2, int row_wrap, int plain, cx<T>* __restrict__ U) {
     constexpr int RH = Spread16Stage<W, T>::RH;
     constexpr int RP = Spread16Stage<W, T>::RP;
@@ -1294,6 +1296,7 @@ spread16_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
     const int s = binstart[bin], e = binstart[bin + 1];
     const TileGeom tg = tile_geom<W>(bin, nbc, BR, BC);
     Spread16Stage<W, T>& st = stg[warp];
+    const int b = blockIdx.y;  // transform
     cx<T>* ub = U + (int64_t)nrows * nf2 * b;
     const bool col_ok = c < tg.TC;
     const int gcol = wrap(tg.tc0 + c, nf2);
@@ -1528,7 +1531,7 @@ template <int W, class T>
 __global__ void __launch_bounds__(128, 4)
 spread_reg_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
                   const int4* __restrict__ slots, int nbusy, int nbc, int BR, int BC, int64_t M,
-                  const double2* __restrict__ fin, int b, int nrows, int nf2, int row_wrap,
+                  const double2* __restrict__ fin, int nrows, int nf2, int row_wrap,
                   int plain, cx<T>* __restrict__ U) {
     using S = typename SpreadRegLayout<W, T>::type;
     constexpr bool kPick = std::is_same_v<S, SpreadPickStage<W, T>>;
@@ -1545,6 +1548,7 @@ spread_reg_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
     const int bin = sl.x, s = sl.y, e = sl.z;
     const TileGeom tg = tile_geom<W>(bin, nbc, BR, BC);
     S& st = reinterpret_cast<S*>(spread_reg_smem)[warp];
+    const int b = blockIdx.y;  // transform
     cx<T>* ub = U + (int64_t)nrows * nf2 * b;
     {
         // lane r: where local row r lands in U
@@ -1707,10 +1711,10 @@ static int launch_interp(const NufftGrid& g, NufftDev& d, double2* f, int B, cud
     const size_t smem = sizeof(cx<T>) * (size_t)tile_elems;
     if (smem > 48 * 1024)
         PF_CUDA(cudaFuncSetAttribute(interp_kernel<W, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    interp_kernel<W, T><<<g.nisb, 128, smem, s>>>(
+    interp_kernel<W, T><<<dim3(g.nisb, B), 128, smem, s>>>(
         d.ipts.as<double2>(), d.iperm.as<int>(), d.binstart.as<int>(), d.iorder.as<int>(), g.nbc,
         g.igroup, g.nsbc, g.bin_rows, g.bin_cols, g.M, d.U.as<cx<T>>(), g.nrows, g.nf2,
-        g.row_wrap, B, f);
+        g.row_wrap, f);
     return check_launch("interp_kernel");
 }
 
@@ -1719,36 +1723,34 @@ static int launch_spread(const NufftGrid& g, NufftDev& d, const double2* f, int 
     // with the deterministic option, one launch per bin colour in a fixed order and plain adds
     const bool col = g.deterministic && g.ncolors > 0;
     const int nl = col ? g.ncolors : 1;
-    for (int b = 0; b < B; ++b) {
-        for (int k = 0; k < nl; ++k) {
-            const int n = col ? g.color_off[k + 1] - g.color_off[k] : g.nbusy;
-            const int* order = col ? d.sorder.as<int>() + g.color_off[k] : d.binorder.as<int>();
-            if (n == 0) continue;
-            if (g.spread_reg && spread_reg_fits(W, g.bin_rows, g.bin_cols)) {
-                constexpr int WR = W <= 10 ? W : 2;
-                const size_t smem = 4 * sizeof(typename SpreadRegLayout<WR, T>::type);
-                if (smem > 48 * 1024)
-                    PF_CUDA(cudaFuncSetAttribute(spread_reg_kernel<WR, T>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                const int4* sl = col ? d.sslot.as<int4>() + g.color_off[k] : d.bslot.as<int4>();
-                spread_reg_kernel<WR, T><<<(n + 3) / 4, 128, smem, s>>>(
-                    d.pts.as<double2>(), d.perm.as<int>(), sl, n, g.nbc, g.bin_rows, g.bin_cols,
-                    g.M, f, b, g.nrows, g.nf2, g.row_wrap, col ? 1 : 0, d.U.as<cx<T>>());
-                PF_TRY(check_launch("spread_reg_kernel"));
-            } else if (W <= 10 && g.bin_cols + W - 1 <= 16) {
-                spread16_kernel<(W <= 10 ? W : 2), T><<<(n + 3) / 4, 128, 0, s>>>(
-                    d.pts.as<double2>(), d.perm.as<int>(), d.binstart.as<int>(), order, n, g.nbc,
-                    g.bin_rows, g.bin_cols, g.M, f, b, g.nrows, g.nf2, g.row_wrap, col ? 1 : 0,
-                    d.U.as<cx<T>>());
-                PF_TRY(check_launch("spread16_kernel"));
-            } else {
-                constexpr int NW = SpreadWarps<W>::N;
-                spread_kernel<W, T><<<(n + NW - 1) / NW, NW * 32, 0, s>>>(
-                    d.pts.as<double2>(), d.perm.as<int>(), d.binstart.as<int>(), order, n, g.nbc,
-                    g.bin_rows, g.bin_cols, g.M, f, b, g.nrows, g.nf2, g.row_wrap, col ? 1 : 0,
-                    d.U.as<cx<T>>());
-                PF_TRY(check_launch("spread_kernel"));
-            }
+    for (int k = 0; k < nl; ++k) {
+        const int n = col ? g.color_off[k + 1] - g.color_off[k] : g.nbusy;
+        const int* order = col ? d.sorder.as<int>() + g.color_off[k] : d.binorder.as<int>();
+        if (n == 0) continue;
+        if (g.spread_reg && spread_reg_fits(W, g.bin_rows, g.bin_cols)) {
+            constexpr int WR = W <= 10 ? W : 2;
+            const size_t smem = 4 * sizeof(typename SpreadRegLayout<WR, T>::type);
+            if (smem > 48 * 1024)
+                PF_CUDA(cudaFuncSetAttribute(spread_reg_kernel<WR, T>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            const int4* sl = col ? d.sslot.as<int4>() + g.color_off[k] : d.bslot.as<int4>();
+            spread_reg_kernel<WR, T><<<dim3((n + 3) / 4, B), 128, smem, s>>>(
+                d.pts.as<double2>(), d.perm.as<int>(), sl, n, g.nbc, g.bin_rows, g.bin_cols,
+                g.M, f, g.nrows, g.nf2, g.row_wrap, col ? 1 : 0, d.U.as<cx<T>>());
+            PF_TRY(check_launch("spread_reg_kernel"));
+        } else if (W <= 10 && g.bin_cols + W - 1 <= 16) {
+            spread16_kernel<(W <= 10 ? W : 2), T><<<dim3((n + 3) / 4, B), 128, 0, s>>>(
+                d.pts.as<double2>(), d.perm.as<int>(), d.binstart.as<int>(), order, n, g.nbc,
+                g.bin_rows, g.bin_cols, g.M, f, g.nrows, g.nf2, g.row_wrap, col ? 1 : 0,
+                d.U.as<cx<T>>());
+            PF_TRY(check_launch("spread16_kernel"));
+        } else {
+            constexpr int NW = SpreadWarps<W>::N;
+            spread_kernel<W, T><<<dim3((n + NW - 1) / NW, B), NW * 32, 0, s>>>(
+                d.pts.as<double2>(), d.perm.as<int>(), d.binstart.as<int>(), order, n, g.nbc,
+                g.bin_rows, g.bin_cols, g.M, f, g.nrows, g.nf2, g.row_wrap, col ? 1 : 0,
+                d.U.as<cx<T>>());
+            PF_TRY(check_launch("spread_kernel"));
         }
     }
     return 0;

@@ -206,7 +206,7 @@ template <int W>
 __global__ void __launch_bounds__(kWarps * 32, W <= 9 ? 6 : W <= 13 ? 5 : 3)
 interp_mma_kernel(const double2* __restrict__ off, const int2* __restrict__ meta,
                   const int4* __restrict__ items, int nitems, const double2* __restrict__ U,
-                  int nrows, int nf2, int row_wrap, double2* __restrict__ f) {
+                  int nrows, int nf2, int row_wrap, int64_t M, double2* __restrict__ f) {
     using H = Shape<W>;
     extern __shared__ __align__(16) unsigned char mma_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -216,6 +216,9 @@ interp_mma_kernel(const double2* __restrict__ off, const int2* __restrict__ meta
     __syncthreads();
     if (slot >= nitems) return;
     const int4 it = items[slot];  // first origin row and column, slots [z, w)
+    // the transform
+    U += (int64_t)nrows * nf2 * blockIdx.y;
+    f += M * blockIdx.y;
     const unsigned never = (unsigned)nrows >> 31;  // 0, which the compiler does not know
     Stage<W>& st = reinterpret_cast<Stage<W>*>(mma_smem)[warp];
     const int t = lane & 3;
@@ -329,7 +332,7 @@ template <int W>
 __global__ void __launch_bounds__(kWarps * 32, W <= 9 ? 5 : W <= 13 ? 4 : 3)
 spread_mma_kernel(const double2* __restrict__ off, const int2* __restrict__ meta,
                   const int4* __restrict__ items, int nitems, const double2* __restrict__ fin,
-                  int nrows, int nf2, int row_wrap, double2* __restrict__ U) {
+                  int nrows, int nf2, int row_wrap, int64_t M, double2* __restrict__ U) {
     using H = Shape<W>;
     extern __shared__ __align__(16) unsigned char mma_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -339,6 +342,9 @@ spread_mma_kernel(const double2* __restrict__ off, const int2* __restrict__ meta
     __syncthreads();
     if (slot >= nitems) return;
     const int4 it = items[slot];  // first origin row and column, slots [z, w)
+    // the transform
+    U += (int64_t)nrows * nf2 * blockIdx.y;
+    fin += M * blockIdx.y;
     const unsigned never = (unsigned)nrows >> 31;  // 0, which the compiler does not know
     SpreadStage<W>& st = reinterpret_cast<SpreadStage<W>*>(mma_smem)[warp];
     const int t = lane & 3, q = lane >> 2;
@@ -450,26 +456,20 @@ template <int W>
 int launch_interp_mma(const NufftGrid& g, NufftDev& d, double2* f, int B, cudaStream_t s) {
     const size_t smem = kWarps * sizeof(Stage<W>);
     PF_TRY(set_smem(interp_mma_kernel<W>, smem));
-    for (int b = 0; b < B; ++b) {
-        interp_mma_kernel<W><<<(g.nitems + kWarps - 1) / kWarps, kWarps * 32, smem, s>>>(
-            d.soff.as<double2>(), d.smeta.as<int2>(), d.items.as<int4>(), g.nitems,
-            d.U.as<double2>() + (int64_t)g.nrows * g.nf2 * b, g.nrows, g.nf2, g.row_wrap, f + g.M * b);
-        PF_TRY(check_launch("interp_mma_kernel"));
-    }
-    return 0;
+    interp_mma_kernel<W><<<dim3((g.nitems + kWarps - 1) / kWarps, B), kWarps * 32, smem, s>>>(
+        d.soff.as<double2>(), d.smeta.as<int2>(), d.items.as<int4>(), g.nitems, d.U.as<double2>(), g.nrows, g.nf2,
+        g.row_wrap, g.M, f);
+    return check_launch("interp_mma_kernel");
 }
 
 template <int W>
 int launch_spread_mma(const NufftGrid& g, NufftDev& d, const double2* f, int B, cudaStream_t s) {
     const size_t smem = kWarps * sizeof(SpreadStage<W>);
     PF_TRY(set_smem(spread_mma_kernel<W>, smem));
-    for (int b = 0; b < B; ++b) {
-        spread_mma_kernel<W><<<(g.nitems + kWarps - 1) / kWarps, kWarps * 32, smem, s>>>(
-            d.soff.as<double2>(), d.smeta.as<int2>(), d.items.as<int4>(), g.nitems, f + g.M * b, g.nrows,
-            g.nf2, g.row_wrap, d.U.as<double2>() + (int64_t)g.nrows * g.nf2 * b);
-        PF_TRY(check_launch("spread_mma_kernel"));
-    }
-    return 0;
+    spread_mma_kernel<W><<<dim3((g.nitems + kWarps - 1) / kWarps, B), kWarps * 32, smem, s>>>(
+        d.soff.as<double2>(), d.smeta.as<int2>(), d.items.as<int4>(), g.nitems, f, g.nrows, g.nf2, g.row_wrap, g.M,
+        d.U.as<double2>());
+    return check_launch("spread_mma_kernel");
 }
 
 template <int W>

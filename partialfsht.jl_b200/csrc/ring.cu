@@ -1163,8 +1163,9 @@ __device__ __forceinline__ void ring_adj_body(const RingTables& t, const RingOut
 template <int RMAX, int NB, bool MIX, bool PHASE>
 __global__ void __launch_bounds__(kAdjWarps * 32)
 ring_adj_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int nitems,
-                const double2* __restrict__ in, double* __restrict__ almd, int b0, int allow_sole) {
+                const double2* __restrict__ in, double* __restrict__ almd, int allow_sole) {
     __shared__ AdjSmem<MIX> sm[kAdjWarps];
+    const int b0 = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int it = blockIdx.x * kAdjWarps + warp;
     if (it >= nitems) return;
@@ -1222,17 +1223,17 @@ static int launch_fwd(const RingTables& t, const RingOut& o, const RingItems& v,
 
 template <int RMAX, int NB, bool MIX>
 static int launch_adj(const RingTables& t, const RingOut& o, const RingItem* items, int nitems,
-                      const double2* in, double2* alm, int b0, int allow_sole, cudaStream_t s) {
-    const int grid = (nitems + kAdjWarps - 1) / kAdjWarps;
+                      const double2* in, double2* alm, int B, int allow_sole, cudaStream_t s) {
+    const dim3 grid((nitems + kAdjWarps - 1) / kAdjWarps, B);
     double* out = reinterpret_cast<double*>(alm);
     if constexpr (!MIX && RMAX <= 4) {
         if (o.phi) {
-            ring_adj_kernel<RMAX, NB, MIX, true><<<grid, kAdjWarps * 32, 0, s>>>(t, o, items, nitems, in, out, b0,
+            ring_adj_kernel<RMAX, NB, MIX, true><<<grid, kAdjWarps * 32, 0, s>>>(t, o, items, nitems, in, out,
                                                                                  allow_sole);
             return check_launch("ring_adj_kernel");
         }
     }
-    ring_adj_kernel<RMAX, NB, MIX, false><<<grid, kAdjWarps * 32, 0, s>>>(t, o, items, nitems, in, out, b0, allow_sole);
+    ring_adj_kernel<RMAX, NB, MIX, false><<<grid, kAdjWarps * 32, 0, s>>>(t, o, items, nitems, in, out, allow_sole);
     return check_launch("ring_adj_kernel");
 }
 
@@ -1274,15 +1275,12 @@ int alm_prepare(double2* alm, int L, int B, const unsigned char* sole_m, int all
 template <bool MIX>
 static int ring_adjoint_t(const RingTables& t, const RingOut& o, const RingItems& it,
                           const double2* in, double2* alm, int B, int allow_sole, cudaStream_t s) {
-    // one pass per transform: the multi-transform shapes share the recurrence but stage NB times
-    // the partial sums per ring through shared memory, the adjoint's co-limit (at lmax 1024,
+    // a transform per row of blocks: the multi-transform shapes share the recurrence but stage NB
+    // times the partial sums per ring through shared memory, the adjoint's co-limit (at lmax 1024,
     // ntrans 4: 0.59 ms with four transforms per pass against 4 x 0.073 ms one by one)
-    for (int b0 = 0; b0 < B; ++b0) {
-        if (it.rmax >= 8) PF_TRY((launch_adj<8, 1, MIX>(t, o, it.items, it.nitems, in, alm, b0, allow_sole, s)));
-        else if (it.rmax >= 4) PF_TRY((launch_adj<4, 1, MIX>(t, o, it.items, it.nitems, in, alm, b0, allow_sole, s)));
-        else PF_TRY((launch_adj<2, 1, MIX>(t, o, it.items, it.nitems, in, alm, b0, allow_sole, s)));
-    }
-    return 0;
+    if (it.rmax >= 8) return launch_adj<8, 1, MIX>(t, o, it.items, it.nitems, in, alm, B, allow_sole, s);
+    if (it.rmax >= 4) return launch_adj<4, 1, MIX>(t, o, it.items, it.nitems, in, alm, B, allow_sole, s);
+    return launch_adj<2, 1, MIX>(t, o, it.items, it.nitems, in, alm, B, allow_sole, s);
 }
 
 // each transform's pass with the items' own tile shape stores the orders covered by a single

@@ -189,7 +189,7 @@ spin_fwd_kernel(SpinTables t, RingOut o, const RingItem* __restrict__ items, int
     if (ptrs) alm = static_cast<const double2*>(ptrs[ptr]);
     const RingItem item = items[it];
     const int m = item.m, am = abs(m);
-    for (int b = 0; b < B; ++b) {
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {  // transforms
         // zeros for the rings the order does not retain (first tile of the order)
         if ((item.flags & kItemFirst) && o.zero_rest) {
             double2* ob = out + o.bstride * b;
@@ -335,7 +335,7 @@ spin_adj_kernel(SpinTables t, RingOut o, const RingItem* __restrict__ items, int
     if (it >= nitems) return;
     if (ptrs) almd = static_cast<double*>(ptrs[ptr]);
     const RingItem item = items[it];
-    for (int b = 0; b < B; ++b) {
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {  // transforms
         const int reff = (item.n + 31) >> 5;
         if (reff >= 3) spin_adj_item<4>(t, o, item, in, almd, b, sm[warp], lane);
         else if (reff == 2) spin_adj_item<2>(t, o, item, in, almd, b, sm[warp], lane);
@@ -390,7 +390,7 @@ int build_spin_items(const std::vector<int>& jlo, const std::vector<int>& jhi, i
 int spin_ring_forward(const SpinTables& t, const RingOut& o, const RingItems& it, const double2* alm,
                       double2* out, int B, cudaStream_t s) {
     if (it.nitems == 0) return 0;
-    spin_fwd_kernel<<<(it.nitems + kSpinWarps - 1) / kSpinWarps, kSpinWarps * 32, 0, s>>>(
+    spin_fwd_kernel<<<dim3((it.nitems + kSpinWarps - 1) / kSpinWarps, std::min(B, 65535)), kSpinWarps * 32, 0, s>>>(
         t, o, it.items, it.nitems, it.jlo, it.jhi, alm, nullptr, 0, out, B);
     return check_launch("spin_fwd_kernel");
 }
@@ -398,7 +398,7 @@ int spin_ring_forward(const SpinTables& t, const RingOut& o, const RingItems& it
 int spin_ring_forward_ptr(const SpinTables& t, const RingOut& o, const RingItems& it,
                           void* const* ptrs, int ptr, double2* out, int B, cudaStream_t s) {
     if (it.nitems == 0) return 0;
-    spin_fwd_kernel<<<(it.nitems + kSpinWarps - 1) / kSpinWarps, kSpinWarps * 32, 0, s>>>(
+    spin_fwd_kernel<<<dim3((it.nitems + kSpinWarps - 1) / kSpinWarps, std::min(B, 65535)), kSpinWarps * 32, 0, s>>>(
         t, o, it.items, it.nitems, it.jlo, it.jhi, nullptr, ptrs, ptr, out, B);
     return check_launch("spin_fwd_kernel");
 }
@@ -409,7 +409,7 @@ int spin_ring_adjoint(const SpinTables& t, const RingOut& o, const RingItems& it
     if (clear)
         PF_CUDA(cudaMemsetAsync(alm, 0, sizeof(double2) * (size_t)(t.lmax + 1) * (2 * t.lmax + 1) * B, s));
     if (it.nitems == 0) return 0;
-    spin_adj_kernel<<<(it.nitems + kSpinAdjWarps - 1) / kSpinAdjWarps, kSpinAdjWarps * 32, 0, s>>>(
+    spin_adj_kernel<<<dim3((it.nitems + kSpinAdjWarps - 1) / kSpinAdjWarps, std::min(B, 65535)), kSpinAdjWarps * 32, 0, s>>>(
         t, o, it.items, it.nitems, in, reinterpret_cast<double*>(alm), nullptr, 0, B);
     return check_launch("spin_adj_kernel");
 }
@@ -417,7 +417,7 @@ int spin_ring_adjoint(const SpinTables& t, const RingOut& o, const RingItems& it
 int spin_ring_adjoint_ptr(const SpinTables& t, const RingOut& o, const RingItems& it,
                           const double2* in, void* const* ptrs, int ptr, int B, cudaStream_t s) {
     if (it.nitems == 0) return 0;
-    spin_adj_kernel<<<(it.nitems + kSpinAdjWarps - 1) / kSpinAdjWarps, kSpinAdjWarps * 32, 0, s>>>(
+    spin_adj_kernel<<<dim3((it.nitems + kSpinAdjWarps - 1) / kSpinAdjWarps, std::min(B, 65535)), kSpinAdjWarps * 32, 0, s>>>(
         t, o, it.items, it.nitems, in, nullptr, ptrs, ptr, B);
     return check_launch("spin_adj_kernel");
 }
