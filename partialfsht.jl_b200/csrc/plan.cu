@@ -243,16 +243,18 @@ void fill_info(pfsht_plan* p) {
 // degrees whose lanes hold R rings costs d (6 R + 4) (the recurrence and the four sums per ring,
 // the transpose-reduce per degree) plus 400 for its start (seed or saved state, ring data, first
 // coefficients: about 60 degrees' work); items are dealt heaviest first to the resident warp
-// slots, and the segment length of 64 q degrees (q = 2..8) with the shortest schedule wins.
-// Measured against fixed lengths at lmax 256 / 1024 / 2048, the adjoint's best lengths were
-// 128 / 128 / 448 degrees (0.021 / 0.066 / 0.263 ms against 0.031 / 0.074 / 0.270 ms at 256),
-// which the model picks.
+// slots (shared by the transforms of an apply), and the segment length of 64 q degrees (q = 1..8)
+// with the shortest schedule wins. Adjoint ring pass against fixed
+// lengths, one transform at lmax 256 / 1024 / 2048: 16.5 / 64.5 / 263.5 us as picked (64 / 128 / 448
+// degrees), 30.5 / 72.3 / 271.1 at 256 degrees; 128 degrees, the shortest length before, took 20.9 at
+// lmax 256. Four transforms at lmax 1024: 213.1 as picked, 220.2 at 128. The model is not exact: its
+// picks were up to 10 percent off the best length (four transforms at lmax 384: 42.8, 38.6 at 192).
 static int choose_segment_degrees(const std::vector<int>& jlo, const std::vector<int>& jhi, int L,
                                   int mmax, int tile, int rmax, int slots) {
     std::vector<double> cost;
     double best = 0.0;
     int best_q = 0;
-    for (int q = 2; q <= 8; ++q) {
+    for (int q = 1; q <= 8; ++q) {
         cost.clear();
         for (int m = 0; m <= std::min(mmax, L); ++m) {
             if (jhi[m] < jlo[m]) continue;
@@ -301,8 +303,9 @@ int build_adjoint_items(pfsht_plan* p, const std::vector<int>& jlo, const std::v
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
         const size_t whole = make_ring_items(jlo, jhi, L, mmax, tile).size();
+        const int slots = std::max(1, sms * 11 / p->B);
         seg = whole >= (size_t)sms * 12 * 8 ? -1
-                                            : choose_segment_degrees(jlo, jhi, L, mmax, tile, rmax, sms * 11);
+                                            : choose_segment_degrees(jlo, jhi, L, mmax, tile, rmax, slots);
     }
     if (seg > 0) {
         PF_TRY(build_ring_segments(p->rt, jlo, jhi, L, mmax, seg, (int64_t)512 << 20, p->adj_seg, s));
