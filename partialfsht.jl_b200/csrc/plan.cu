@@ -509,6 +509,25 @@ int plan_create(const double* theta, const double* phi, int64_t npts, int lmax, 
 // point sets from this size on are planned by the device scans (planner_dev.cu)
 constexpr int64_t kDevicePlannerMin = 1 << 15;
 
+// the boxes' events, and the adjoint's coefficient scratch: an array for each box after the first,
+// within 256 MB, and one where that much cannot be had
+int alloc_box_sums(pfsht_plan* p, int nb) {
+    for (int i = 0; i <= nb; ++i) {
+        cudaEvent_t e;
+        PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        p->ev_box.push_back(e);
+    }
+    if (nb < 2) return 0;
+    const size_t bytes = sizeof(double2) * (size_t)(p->L + 1) * (2 * p->L + 1) * p->B;
+    p->nacc = (int)std::max<size_t>(1, std::min<size_t>(nb - 1, ((size_t)256 << 20) / bytes));
+    if (p->nacc > 1) {
+        if (p->acc.alloc(bytes * p->nacc) == 0) return 0;
+        (void)cudaGetLastError();  // not for the next launch's check
+    }
+    p->nacc = 1;
+    return p->acc.alloc(bytes);
+}
+
 // MultiBoxLeaf (src/MultiBox.jl:32-66): one stretched-leaf plan per group of the partition
 int build_multibox(pfsht_plan* p, const Partition& part, const double* th, const double* ph,
                    int precision, const pfsht_opts& o) {
@@ -539,8 +558,7 @@ int build_multibox(pfsht_plan* p, const Partition& part, const double* th, const
     p->precision = p->boxes[0]->precision;
     PF_TRY(upload(p->gidx, idx, p->st_stream));
     PF_TRY(p->fg.alloc(sizeof(double2) * (size_t)p->M * p->B));
-    if (nb > 1) PF_TRY(p->acc.alloc(sizeof(double2) * (size_t)(p->L + 1) * (2 * p->L + 1) * p->B));
-    return 0;
+    return alloc_box_sums(p, nb);
 }
 
 // the same from a partition computed on the device: each box's points are gathered on the device
@@ -585,7 +603,7 @@ int build_multibox_device(pfsht_plan* p, const DevPartition& part, const double*
     }
     p->precision = p->boxes[0]->precision;
     PF_TRY(p->fg.alloc(sizeof(double2) * (size_t)p->M * p->B));
-    if (nb > 1) PF_TRY(p->acc.alloc(sizeof(double2) * (size_t)(p->L + 1) * (2 * p->L + 1) * p->B));
+    PF_TRY(alloc_box_sums(p, nb));
     PF_CUDA(cudaStreamSynchronize(s));
     return 0;
 }
@@ -625,34 +643,67 @@ unsigned grid_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<in
 int apply_forward(pfsht_plan* p, const double2* alm, double2* f, cudaStream_t s);
 int apply_adjoint(pfsht_plan* p, const double2* f, double2* alm, cudaStream_t s);
 
-int multibox_forward(pfsht_plan* p, const double2* alm, double2* f, cudaStream_t s) {
+// The boxes are independent, and each alone is a chain of launches that fills little of the GPU: box 0
+// runs on the caller's stream, the others on streams of their own, forked from it and joined to it by
+// events (two 512-degree caps, both directions: 211 us one after the other, 132 side by side).
+int multibox_forward_boxes(pfsht_plan* p, const double2* alm, double2* f, cudaStream_t s) {
+    PF_CUDA(cudaEventRecord(p->ev_box[0], s));
     for (size_t i = 0; i < p->boxes.size(); ++i) {
         const int64_t mb = p->box_off[i + 1] - p->box_off[i];
         double2* fgi = p->fg.as<double2>() + p->B * p->box_off[i];
-        PF_TRY(apply_forward(p->boxes[i].get(), alm, fgi, s));
-        box_scatter_kernel<<<grid_for(mb * p->B), 256, 0, s>>>(
+        cudaStream_t si = i == 0 ? s : p->boxes[i]->st_stream;
+        if (i > 0) PF_CUDA(cudaStreamWaitEvent(si, p->ev_box[0], 0));
+        PF_TRY(apply_forward(p->boxes[i].get(), alm, fgi, si));
+        box_scatter_kernel<<<grid_for(mb * p->B), 256, 0, si>>>(
             fgi, p->gidx.as<int>() + p->box_off[i], mb, p->M, p->B, f);
         PF_TRY(check_launch("box_scatter_kernel"));
+        if (i > 0) PF_CUDA(cudaEventRecord(p->ev_box[i + 1], si));
+    }
+    for (size_t i = 1; i < p->boxes.size(); ++i) PF_CUDA(cudaStreamWaitEvent(s, p->ev_box[i + 1], 0));
+    return 0;
+}
+
+int multibox_adjoint_boxes(pfsht_plan* p, const double2* f, double2* alm, cudaStream_t s) {
+    const int64_t nc = (int64_t)(p->L + 1) * (2 * p->L + 1) * p->B;
+    PF_CUDA(cudaEventRecord(p->ev_box[0], s));
+    // each box's adjoint overwrites its output: the first writes alm, the others the coefficient
+    // scratch arrays in turn, which are added to alm in the boxes' order
+    for (size_t i = 0; i < p->boxes.size(); ++i) {
+        const int64_t mb = p->box_off[i + 1] - p->box_off[i];
+        double2* fgi = p->fg.as<double2>() + p->B * p->box_off[i];
+        cudaStream_t si = i == 0 ? s : p->boxes[i]->st_stream;
+        // a scratch array is free once the box that used it before has been added
+        if (i > 0) PF_CUDA(cudaStreamWaitEvent(si, p->ev_box[(int)i <= p->nacc ? 0 : i - p->nacc + 1], 0));
+        box_gather_kernel<<<grid_for(mb * p->B), 256, 0, si>>>(
+            f, p->gidx.as<int>() + p->box_off[i], mb, p->M, p->B, fgi);
+        PF_TRY(check_launch("box_gather_kernel"));
+        double2* acc = i == 0 ? alm : p->acc.as<double2>() + nc * (int64_t)((i - 1) % p->nacc);
+        PF_TRY(apply_adjoint(p->boxes[i].get(), fgi, acc, si));
+        if (i == 0) continue;
+        PF_CUDA(cudaEventRecord(p->ev_box[i + 1], si));
+        PF_CUDA(cudaStreamWaitEvent(s, p->ev_box[i + 1], 0));
+        coeff_add_kernel<<<grid_for(nc), 256, 0, s>>>(alm, acc, nc);
+        PF_TRY(check_launch("coeff_add_kernel"));
+        PF_CUDA(cudaEventRecord(p->ev_box[i + 1], s));
     }
     return 0;
 }
 
+// after an error part way, the caller's stream still waits for what the boxes' streams were given
+int multibox_join(pfsht_plan* p, int rc, cudaStream_t s) {
+    if (rc != 0)
+        for (size_t i = 1; i < p->boxes.size(); ++i)
+            if (cudaEventRecord(p->ev_box[i + 1], p->boxes[i]->st_stream) == cudaSuccess)
+                (void)cudaStreamWaitEvent(s, p->ev_box[i + 1], 0);
+    return rc;
+}
+
+int multibox_forward(pfsht_plan* p, const double2* alm, double2* f, cudaStream_t s) {
+    return multibox_join(p, multibox_forward_boxes(p, alm, f, s), s);
+}
+
 int multibox_adjoint(pfsht_plan* p, const double2* f, double2* alm, cudaStream_t s) {
-    const int64_t nc = (int64_t)(p->L + 1) * (2 * p->L + 1) * p->B;
-    for (size_t i = 0; i < p->boxes.size(); ++i) {
-        const int64_t mb = p->box_off[i + 1] - p->box_off[i];
-        double2* fgi = p->fg.as<double2>() + p->B * p->box_off[i];
-        box_gather_kernel<<<grid_for(mb * p->B), 256, 0, s>>>(
-            f, p->gidx.as<int>() + p->box_off[i], mb, p->M, p->B, fgi);
-        PF_TRY(check_launch("box_gather_kernel"));
-        // each box's adjoint overwrites its output: the first writes alm, the others are added
-        PF_TRY(apply_adjoint(p->boxes[i].get(), fgi, i == 0 ? alm : p->acc.as<double2>(), s));
-        if (i > 0) {
-            coeff_add_kernel<<<grid_for(nc), 256, 0, s>>>(alm, p->acc.as<double2>(), nc);
-            PF_TRY(check_launch("coeff_add_kernel"));
-        }
-    }
-    return 0;
+    return multibox_join(p, multibox_adjoint_boxes(p, f, alm, s), s);
 }
 
 int plan_create(const double* theta, const double* phi, int64_t npts, int lmax, int ntrans,

@@ -73,10 +73,13 @@ struct pfsht_plan {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // MultiBox (src/MultiBox.jl): one stretched-leaf plan per box; gidx holds the boxes' point
     // indices one box after the other (box i at [box_off[i], box_off[i + 1])), fg the boxes'
-    // fields in the same order (box i at B box_off[i]), acc one coefficient array for the sum
+    // fields in the same order (box i at B box_off[i]), acc nacc coefficient arrays for the sum; the
+    // boxes' events: ev_box[0] the fork, ev_box[i + 1] box i's end
     std::vector<std::unique_ptr<pfsht_plan>> boxes;
     std::vector<int64_t> box_off;
     DevBuf gidx, fg, acc;
+    int nacc = 1;
+    std::vector<cudaEvent_t> ev_box;
     pfsht_plan_info info{};
     StageClock clk;
     // solve!'s workspace where it is small (solve.cu), the pinned copies of its state and their events
@@ -98,6 +101,7 @@ struct pfsht_plan {
                               ev_fwd_done, ev_f_in_ready, ev_copied})
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : ev_blk) cudaEventDestroy(e);
+        for (cudaEvent_t e : ev_box) cudaEventDestroy(e);
         for (cudaEvent_t e : clk.ev) cudaEventDestroy(e);
         for (cudaEvent_t e : solve_ev)
             if (e) cudaEventDestroy(e);
