@@ -1160,8 +1160,13 @@ __device__ __forceinline__ void ring_adj_body(const RingTables& t, const RingOut
     }
 }
 
+// FP64 at four rings a lane: 16 one-warp blocks per SM, i.e. 128 registers instead of the 164 that the
+// compiler takes for itself (12 blocks). The pass is bound by shared-memory wavefronts (76 percent of
+// their peak, FP64 55) and by the latency that so few warps leave open: at lmax 1024 / 2048, 64.5 to
+// 62.3 and 263.5 to 249.2 us, four transforms at 1024 213 to 202. Sums over the lanes without shared
+// memory (butterflies of the lanes, at the same registers) took 68.5 and 288 us, 18 blocks (spills) 261.
 template <int RMAX, int NB, bool MIX, bool PHASE>
-__global__ void __launch_bounds__(kAdjWarps * 32)
+__global__ void __launch_bounds__(kAdjWarps * 32, RMAX == 4 && !MIX ? 16 : 1)
 ring_adj_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int nitems,
                 const double2* __restrict__ in, double* __restrict__ almd, int allow_sole) {
     __shared__ AdjSmem<MIX> sm[kAdjWarps];
@@ -1525,8 +1530,6 @@ static int fwd_batch_shape(const RingSlot* slots, const RingBatchGroup& g, void*
 template <bool MIX>
 static int adj_batch_shape(const RingSlot* slots, const RingBatchGroup& g, void* const* ptrs,
                            cudaStream_t s) {
-    if (g.nb == 4) return launch_adj_batch<1, 4, MIX>(slots, g, ptrs, s);
-    if (g.nb == 2) return launch_adj_batch<2, 2, MIX>(slots, g, ptrs, s);
     if (g.rmax >= 8) return launch_adj_batch<8, 1, MIX>(slots, g, ptrs, s);
     if (g.rmax >= 4) return launch_adj_batch<4, 1, MIX>(slots, g, ptrs, s);
     return launch_adj_batch<2, 1, MIX>(slots, g, ptrs, s);
