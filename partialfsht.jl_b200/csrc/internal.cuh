@@ -262,6 +262,9 @@ struct SpinTablesOwner {
 // tables of a ring set (ring colatitudes theta_rings; reflect: the rings stand for pi - theta)
 int build_spin_tables(const std::vector<double>& theta_rings, bool reflect, int lmax, int spin,
                       SpinTablesOwner& own, cudaStream_t s);
+// rings per item for a plan of B transforms
+int spin_tile(const std::vector<int>& jlo, const std::vector<int>& jhi, int lmax, int spin, int B,
+              bool deterministic);
 // items over (m = -lmax..lmax, tiles of rings_per_tile retained rings), heaviest first; jlo/jhi
 // indexed by |m| (uploaded into own.jlo / own.jhi)
 int build_spin_items(const std::vector<int>& jlo, const std::vector<int>& jhi, int lmax, int spin,

@@ -18,8 +18,9 @@
 // Forward: each ring accumulates N_l a_{lm} d_l and writes G (windowed, mirrored into the DFS
 // rows with sign (-1)^(m+s), zeros for the rings the order does not retain).
 // Adjoint: each ring scales its G value by its window and 2^E once per exponent change; per
-// degree the lanes' partial sums are transposed through shared memory and reduced one degree per
-// lane, then added into the coefficient (orders split over several tiles add atomically).
+// degree the lanes' partial sums are staged in shared memory, and every 16 degrees a lane sums the
+// real or imaginary part of one of them and adds it into the coefficient (orders split over several
+// tiles add atomically).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -33,7 +34,11 @@ namespace pf {
 namespace {
 
 constexpr int kSpinWarps = 4;     // forward: warps per block
-constexpr int kSpinAdjWarps = 2;  // adjoint: warps per block (18 KB of shared memory each)
+constexpr int kSpinAdjWarps = 1;  // adjoint: warps per block (a finer tail)
+// Adjoint: blocks per SM, 128 registers a thread and 9 KB of shared memory a warp. Sums staged 32
+// degrees at a time (18 KB, 168 registers) left 12 warps: at lmax 1024 134 against 127 us, two
+// transforms 218 against 201, a lmax 1536 patch 587 against 513.
+constexpr int kSpinAdjBlocks = 16;
 constexpr int kSpinFwdUnroll = 4;  // forward degree loop (measured: 0.357 ms vs 0.370 unrolled by 8)
 
 struct SpinCoef {
@@ -209,7 +214,7 @@ spin_fwd_kernel(SpinTables t, RingOut o, const RingItem* __restrict__ items, int
 
 struct SpinAdjSmem {
     SpinCoef c[32];
-    double2 red[32][33];
+    double red[32][33];  // (degree, re / im) rows of 16 degrees, a partial sum per lane
 };
 
 template <int R>
@@ -276,39 +281,40 @@ __device__ void spin_adj_item(const SpinTables& t, const RingOut& o, const RingI
             p.x = fma(dn, gs[r].x, p.x);
             p.y = fma(dn, gs[r].y, p.y);
         }
-        sm.red[i][lane] = p;
+        sm.red[2 * (i & 15)][lane] = p.x;
+        sm.red[2 * (i & 15) + 1][lane] = p.y;
     };
     for (int lb = l0 + 1; lb <= L; lb += 32) {
         const int nl = min(32, L - lb + 1);
         __syncwarp();
         if (lane < nl) sm.c[lane] = spin_coef(t.lt, lb + lane, m, n);
         __syncwarp();
-        if (nl == 32) {
-#pragma unroll 8
-            for (int i = 0; i < 32; ++i) step(i);
-        } else {
-            for (int i = 0; i < nl; ++i) step(i);
-        }
-        __syncwarp();
-        if (lane < nl) {
-            double sx0 = 0.0, sy0 = 0.0, sx1 = 0.0, sy1 = 0.0;
-#pragma unroll 8
-            for (int q = 0; q < 32; q += 2) {
-                const double2 v0 = sm.red[lane][q], v1 = sm.red[lane][q + 1];
-                sx0 += v0.x;
-                sy0 += v0.y;
-                sx1 += v1.x;
-                sy1 += v1.y;
-            }
-            const double N = sm.c[lane].N;
-            const size_t e = 2 * sidx(lb + lane, m, L);
-            if (item.flags & kItemSole) {
-                ad[e] = (sx0 + sx1) * N;
-                ad[e + 1] = (sy0 + sy1) * N;
+        for (int h = 0; h < nl; h += 16) {
+            const int cnt = min(16, nl - h);
+            if (cnt == 16) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) step(h + i);
             } else {
-                atomicAdd(ad + e, (sx0 + sx1) * N);
-                atomicAdd(ad + e + 1, (sy0 + sy1) * N);
+                for (int i = 0; i < cnt; ++i) step(h + i);
             }
+            __syncwarp();
+            if (lane < 2 * cnt) {
+                // four independent partial sums: the chain of dependent adds is 8 long, not 32
+                double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+                for (int q = 0; q < 32; q += 4) {
+                    s0 += sm.red[lane][q];
+                    s1 += sm.red[lane][q + 1];
+                    s2 += sm.red[lane][q + 2];
+                    s3 += sm.red[lane][q + 3];
+                }
+                const int i = h + (lane >> 1);
+                const double v = ((s0 + s1) + (s2 + s3)) * sm.c[i].N;
+                double* dst = ad + 2 * sidx(lb + i, m, L) + (lane & 1);
+                if (item.flags & kItemSole) *dst = v;
+                else atomicAdd(dst, v);
+            }
+            __syncwarp();
         }
         // renormalise every 32 degrees (exact powers of two); the scaled ring values follow E
 #pragma unroll
@@ -325,7 +331,7 @@ __device__ void spin_adj_item(const SpinTables& t, const RingOut& o, const RingI
     }
 }
 
-__global__ void __launch_bounds__(kSpinAdjWarps * 32)
+__global__ void __launch_bounds__(kSpinAdjWarps * 32, kSpinAdjBlocks)
 spin_adj_kernel(SpinTables t, RingOut o, const RingItem* __restrict__ items, int nitems,
                 const double2* __restrict__ in, double* __restrict__ almd, void* const* __restrict__ ptrs,
                 int ptr, int B) {
@@ -344,6 +350,28 @@ spin_adj_kernel(SpinTables t, RingOut o, const RingItem* __restrict__ items, int
 }
 
 }  // namespace
+
+// Rings per item. An item is one warp's whole order, and small plans have fewer of them than the GPU
+// runs at a time: tiles of 128 rings (four a lane, the fewest instructions per ring) are halved while
+// there are less than eight items per SM, down to one ring a lane. Forward and
+// adjoint pass at lmax 256: 22.3 and 32.8 us in tiles of 128 rings, 15.9 and 25.4 in tiles of 32; at
+// lmax 512 38.3 and 60.4 against 28.2 and 47.7; at lmax 1024 (2000 items of 128 rings) 128.6 against
+// 153 and 211 in tiles of 64 and 32, adjoint.
+// The adjoint adds an order's tiles atomically: a deterministic plan keeps 128 rings.
+int spin_tile(const std::vector<int>& jlo, const std::vector<int>& jhi, int lmax, int spin, int B,
+              bool deterministic) {
+    int tile = 128;
+    auto count = [&](int t) {
+        int64_t n = 0;
+        for (int m = -lmax; m <= lmax; ++m) {
+            const int am = std::abs(m);
+            if (std::max(am, std::abs(spin)) <= lmax && jlo[am] <= jhi[am]) n += (jhi[am] - jlo[am] + t) / t;
+        }
+        return n * B;
+    };
+    while (!deterministic && tile > 32 && count(tile) < 148 * 8) tile /= 2;
+    return tile;
+}
 
 int build_spin_items(const std::vector<int>& jlo, const std::vector<int>& jhi, int lmax, int spin,
                      int rings_per_tile, RingItemsOwner& own, cudaStream_t s) {
