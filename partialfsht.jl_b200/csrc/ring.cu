@@ -1160,13 +1160,14 @@ __device__ __forceinline__ void ring_adj_body(const RingTables& t, const RingOut
     }
 }
 
-// FP64 at four rings a lane: 16 one-warp blocks per SM, i.e. 128 registers instead of the 164 that the
-// compiler takes for itself (12 blocks). The pass is bound by shared-memory wavefronts (76 percent of
+// Up to four rings a lane: 16 one-warp blocks per SM, i.e. 128 registers instead of the 164 that the
+// compiler takes for itself in FP64 (12 blocks); the FP32 sums fit without (126), but take more when
+// one block is asked for (lmax 2048, both directions: 764 against 727 us). The pass is bound by shared-memory wavefronts (76 percent of
 // their peak, FP64 55) and by the latency that so few warps leave open: at lmax 1024 / 2048, 64.5 to
 // 62.3 and 263.5 to 249.2 us, four transforms at 1024 213 to 202. Sums over the lanes without shared
 // memory (butterflies of the lanes, at the same registers) took 68.5 and 288 us, 18 blocks (spills) 261.
 template <int RMAX, int NB, bool MIX, bool PHASE>
-__global__ void __launch_bounds__(kAdjWarps * 32, RMAX == 4 && !MIX ? 16 : 1)
+__global__ void __launch_bounds__(kAdjWarps * 32, RMAX <= 4 ? 16 : 8)
 ring_adj_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int nitems,
                 const double2* __restrict__ in, double* __restrict__ almd, int allow_sole) {
     __shared__ AdjSmem<MIX> sm[kAdjWarps];
