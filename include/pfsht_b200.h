@@ -227,7 +227,7 @@ typedef enum {
 /* Conjugate gradients on (A^H W A + C^-1) alm = A^H W f on the device: f and alm are device
  * arrays in the plan's layouts (alm is overwritten with the solution); prior is a host array of
  * lmax + 1 values C_l (WIENER only, NULL otherwise); w is a device array of npts point weights or
- * NULL. Each iteration is one CUDA graph with device-side scalars; the updates freeze where the
+ * NULL. Scalars stay on the device; the updates freeze where the
  * reference's loop breaks. *iters and *relres are the reference's info.iters and info.relres. */
 pfsht_status pfsht_solve(pfsht_plan* plan, const void* f, void* alm, int32_t mode, double rtol,
                          int32_t maxiter, const double* prior, const double* w, void* stream,

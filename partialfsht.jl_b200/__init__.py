@@ -614,8 +614,8 @@ _SOLVE_MODES = {"cg": 0, "wiener": 1, "minnorm": 2}
 
 def solve(alm, plan, f, *, mode="cg", rtol=1e-6, maxiter=500, prior=None, w=None, stream=None):
     """solve!(alm, plan, f; mode, rtol, maxiter, prior, w) (src/Analysis.jl:375-436):
-    conjugate gradients on (A^H W A + C^-1) alm = A^H W f, run on the device (one CUDA graph per
-    iteration, scalars on the device). ``alm`` (overwritten) and ``f`` are CUDA tensors or host
+    conjugate gradients on (A^H W A + C^-1) alm = A^H W f, run on the device (the workspace
+    is kept with the plan, scalars on the device). ``alm`` (overwritten) and ``f`` are CUDA tensors or host
     arrays; ``prior`` is C_l for l = 0..lmax ("wiener" only); ``w`` per-point weights. Returns
     (alm, info) with info's mode, iters, relres, shannon and Δℓ."""
     if mode not in _SOLVE_MODES:
