@@ -406,6 +406,10 @@ int setup_cols(NufftGrid& g, NufftDev& d, int B, cudaStream_t s) {
     if (g.fp32 || !g.gap_ok || g.row_wrap || cols_per_block(g, B) < 1 || !make_fft(g.n1, th) || !make_fft(g.nf1, f1) ||
         g.nf1 < g.n1 || (int64_t)g.nf1 * 8 > 65535 || (int64_t)g.nf1 * g.ncols > kColsMostCells)
         return 0;
+    // the limit belongs to the kernels, not to a plan: it is the same for every plan and set before any
+    // launch, since a plan that set its own size before a launch could lower it under another thread's
+    PF_CUDA(cudaFuncSetAttribute(cols_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+    PF_CUDA(cudaFuncSetAttribute(cols_adj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
     PF_TRY(upload_roots(g.n1, d.roots_th, s));
     PF_TRY(upload_roots(g.nf1, d.roots_f1, s));
     g.cols = 1;
@@ -415,7 +419,6 @@ int setup_cols(NufftGrid& g, NufftDev& d, int B, cudaStream_t s) {
 int cols_forward(const NufftGrid& g, NufftDev& d, const double2* H, int B, int iflag, cudaStream_t s) {
     Cols c;
     const int smem = fill_cols(g, d, B, c);
-    PF_CUDA(cudaFuncSetAttribute(cols_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const int zeros = g.gap_hi > g.gap_lo ? g.nrows : 0;
     cols_fwd_kernel<<<dim3(c.nblocks + zeros, B), block_threads(c.C, c.f1.n), smem, s>>>(c, H, d.U.as<double2>(), -1.0,
                                                                        iflag > 0 ? 1.0 : -1.0);
@@ -425,7 +428,6 @@ int cols_forward(const NufftGrid& g, NufftDev& d, const double2* H, int B, int i
 int cols_adjoint(const NufftGrid& g, NufftDev& d, double2* H, int B, int iflag, cudaStream_t s) {
     Cols c;
     const int smem = fill_cols(g, d, B, c);
-    PF_CUDA(cudaFuncSetAttribute(cols_adj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cols_adj_kernel<<<dim3(c.nblocks, B), block_threads(c.C, c.f1.n), smem, s>>>(c, d.U.as<double2>(), H, 1.0, iflag > 0 ? 1.0 : -1.0);
     return check_launch("cols_adj_kernel");
 }
