@@ -1681,6 +1681,23 @@ spread_reg_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
 }
 #undef PF_ROW_PAIR_CASES
 
+// Dynamic shared memory past the default 48 KB: the kernel's limit goes to the most that the device
+// has, whatever the plan's bytes, since it belongs to the kernel and a thread with a smaller plan
+// could lower it between another thread's setting and its launch. More than that is refused.
+template <class K>
+static int allow_smem(K kernel, size_t bytes) {
+    if (bytes <= 48 * 1024) return 0;
+    cudaFuncAttributes a;
+    int dev = 0, most = 0;
+    PF_CUDA(cudaFuncGetAttributes(&a, kernel));
+    PF_CUDA(cudaGetDevice(&dev));
+    PF_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    most -= (int)a.sharedSizeBytes;
+    PF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)std::max<size_t>(bytes, most)));
+    return 0;
+}
+
 // groups per resident block from which the one-transform interpolation is pipelined
 constexpr int kInterpPipeGroups = 4;
 
@@ -1689,9 +1706,7 @@ static int launch_interp(const NufftGrid& g, NufftDev& d, double2* f, int B, cud
     const int tile_elems = (g.bin_rows + W - 1) * ((g.igroup * g.bin_cols + W - 1) | 1);
     if (B == 1 && g.interp_pipe && g.igroup * g.bin_cols + W - 1 <= 32 && g.nisb > 0) {
         const size_t smem2 = 2 * sizeof(cx<T>) * (size_t)tile_elems;
-        if (smem2 > 48 * 1024)
-            PF_CUDA(cudaFuncSetAttribute(interp_pipe_kernel<W, T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+        PF_TRY(allow_smem(interp_pipe_kernel<W, T>, smem2));
         int per = 0, dev = 0, nsm = 0;
         PF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, interp_pipe_kernel<W, T>, 128, smem2));
         PF_CUDA(cudaGetDevice(&dev));
@@ -1709,8 +1724,7 @@ static int launch_interp(const NufftGrid& g, NufftDev& d, double2* f, int B, cud
         }
     }
     const size_t smem = sizeof(cx<T>) * (size_t)tile_elems;
-    if (smem > 48 * 1024)
-        PF_CUDA(cudaFuncSetAttribute(interp_kernel<W, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PF_TRY(allow_smem(interp_kernel<W, T>, smem));
     interp_kernel<W, T><<<dim3(g.nisb, B), 128, smem, s>>>(
         d.ipts.as<double2>(), d.iperm.as<int>(), d.binstart.as<int>(), d.iorder.as<int>(), g.nbc,
         g.igroup, g.nsbc, g.bin_rows, g.bin_cols, g.M, d.U.as<cx<T>>(), g.nrows, g.nf2,

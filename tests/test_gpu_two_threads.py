@@ -62,3 +62,12 @@ def test_column_kernels(pf, O, cuda, sizes):
     plans = [pf.Plan(*cap_points(1500, theta_star=t, rng=rng), lmax=L, tol=1e-8, method="stretch", fft_lengths=n)
              for L, t, n in sizes]
     apply_from_two_threads(pf, O, plans, 2)
+
+
+# interpolation tiles of 57 and 110 KB
+@pytest.mark.parametrize("rows", [(100, 200)])
+def test_interpolation_tiles(pf, O, cuda, rows):
+    rng = np.random.default_rng(3)
+    plans = [pf.Plan(*cap_points(1500, theta_star=0.35, rng=rng), lmax=256, tol=1e-8, method="stretch",
+                     fft_lengths="minimal", bin_rows=r) for r in rows]
+    apply_from_two_threads(pf, O, plans, 4)
