@@ -108,7 +108,7 @@ typedef struct pfsht_plan_info {
     /* NUFFT */
     int32_t nufft_w, nf1, nf2, row0, nrows, ncols;
     double nufft_beta;
-    int64_t device_bytes; /* device memory the plan holds */
+    int64_t device_bytes; /* device memory the plan holds when asked */
     int32_t spin;         /* spin weight */
     int32_t pad_;
 } pfsht_plan_info;

@@ -182,12 +182,7 @@ void fill_info(pfsht_plan* p) {
     in.tol = p->tol;
     in.spin = p->spin;
     if (p->kind == kMultiBox) {
-        for (const auto& c : p->boxes) {
-            in.ring_work += c->info.ring_work;
-            in.device_bytes += c->info.device_bytes;
-        }
-        in.device_bytes += (int64_t)(p->gidx.bytes + p->fg.bytes + p->acc.bytes + p->st_alm.bytes +
-                                     p->st_f.bytes + p->st_alm2.bytes + p->st_f2.bytes);
+        for (const auto& c : p->boxes) in.ring_work += c->info.ring_work;
         return;
     }
     if (p->kind == kDirect) {
@@ -219,17 +214,6 @@ void fill_info(pfsht_plan* p) {
         in.nrows = p->ng.nrows;
         in.ncols = p->ng.ncols;
     }
-    int64_t bytes = 0;
-    for (const DevBuf* b : {&p->cos_t, &p->log2sin, &p->log2c, &p->w, &p->ab, &p->aboff, &p->fwd_items.items, &p->adj_items.items,
-                            &p->adj_seg.ck_p, &p->adj_seg.ck_E, &p->fwd_seg.ck_p, &p->fwd_seg.ck_E, &p->fwd_items.blocks,
-                            &p->H, &p->direct_parts, &p->phi_pts, &p->nd.pts, &p->nd.perm, &p->nd.binstart,
-                            &p->nd.binorder, &p->nd.sorder, &p->nd.bslot, &p->nd.sslot,
-                            &p->nd.iorder, &p->nd.items, &p->nd.soff, &p->nd.smeta, &p->nd.ipts, &p->nd.iperm, &p->nd.counter,
-                            &p->nd.roots_th, &p->nd.roots_f1, &p->nd.colp2, &p->nd.p2col, &p->nd.mult1, &p->nd.dec2, &p->nd.pad,
-                            &p->nd.U, &p->st_alm, &p->st_f, &p->ab_fwd, &p->st_alm2,
-                            &p->st_f2, &p->blk_fwd_items, &p->blk_adj_items})
-        bytes += (int64_t)b->bytes;
-    in.device_bytes = bytes;
 }
 
 // Adjoint items: tiles of 32 * R rings whose sums add atomically when an order spans several;
@@ -913,6 +897,24 @@ int apply_adjoint(pfsht_plan* p, const double2* f, double2* alm, cudaStream_t s)
 
 namespace pf {
 
+// Device memory the plan holds now: the staging of host arrays, a batch's field and column array and a
+// solve's kept workspace come after the build.
+int64_t plan_bytes(const pfsht_plan* p) {
+    int64_t bytes = 0;
+    for (const DevBuf* b : {&p->cos_t, &p->log2sin, &p->log2c, &p->w, &p->ab, &p->aboff, &p->fwd_items.items, &p->adj_items.items,
+                            &p->adj_seg.ck_p, &p->adj_seg.ck_E, &p->fwd_seg.ck_p, &p->fwd_seg.ck_E, &p->fwd_items.blocks,
+                            &p->H, &p->direct_parts, &p->phi_pts, &p->nd.pts, &p->nd.perm, &p->nd.binstart,
+                            &p->nd.binorder, &p->nd.sorder, &p->nd.bslot, &p->nd.sslot,
+                            &p->nd.iorder, &p->nd.items, &p->nd.soff, &p->nd.smeta, &p->nd.ipts, &p->nd.iperm, &p->nd.counter,
+                            &p->nd.roots_th, &p->nd.roots_f1, &p->nd.colp2, &p->nd.p2col, &p->nd.mult1, &p->nd.dec2, &p->nd.pad,
+                            &p->nd.U, &p->st_alm, &p->st_f, &p->ab_fwd, &p->st_alm2,
+                            &p->st_f2, &p->blk_fwd_items, &p->blk_adj_items, &p->solve_ws,
+                            &p->gidx, &p->fg, &p->acc})
+        bytes += (int64_t)b->bytes;
+    for (const auto& c : p->boxes) bytes += plan_bytes(c.get());
+    return bytes;
+}
+
 int plan_forward_after_ring(pfsht_plan* p, double2* f, cudaStream_t s) {
     StageClock* clk = &p->clk;
     if (p->kind == kDirect) {
@@ -1425,10 +1427,11 @@ int64_t pfsht_ring_work(const pfsht_plan* p) { return p ? p->info.ring_work : -1
 pfsht_status pfsht_plan_get_info(const pfsht_plan* p, pfsht_plan_info* info) {
     if (!p || !info) return (pfsht_status)fail(PFSHT_ERR_ARGUMENT, "NULL argument");
     *info = p->info;
+    info->device_bytes = plan_bytes(p);
     return PFSHT_OK;
 }
 
-int64_t pfsht_workspace_bytes(const pfsht_plan* p) { return p ? p->info.device_bytes : -1; }
+int64_t pfsht_workspace_bytes(const pfsht_plan* p) { return p ? plan_bytes(p) : -1; }
 
 int32_t pfsht_plan_num_boxes(const pfsht_plan* p) {
     if (!p) return -1;
@@ -1440,13 +1443,13 @@ pfsht_status pfsht_plan_box(const pfsht_plan* p, int32_t box, pfsht_plan_info* i
     const int32_t nb = pfsht_plan_num_boxes(p);
     if (box < 0 || box >= nb) return (pfsht_status)fail(PFSHT_ERR_ARGUMENT, "box index out of range");
     if (p->kind != kMultiBox) {
-        if (info) *info = p->info;
+        if (info) pfsht_plan_get_info(p, info);
         if (indices)
             for (int64_t i = 0; i < p->M; ++i) indices[i] = i;
         return PFSHT_OK;
     }
     const pfsht_plan* c = p->boxes[box].get();
-    if (info) *info = c->info;
+    if (info) pfsht_plan_get_info(c, info);
     if (indices) {
         const int64_t mb = p->box_off[box + 1] - p->box_off[box];
         std::vector<int32_t> h(mb);

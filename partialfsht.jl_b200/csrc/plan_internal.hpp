@@ -139,6 +139,7 @@ int plan_host_enqueue(pfsht_plan* p, const void* in, void* out, bool fwd, cudaSt
                       bool order_on_s = true, bool zero_async = false);
 // wait for the plan's asynchronous padding zeroing, if one is running
 void plan_host_wait(pfsht_plan* p);
+int64_t plan_bytes(const pfsht_plan* p);  // device memory the plan holds now
 // allocate the plan's staging buffers for host-buffer applies
 int plan_host_staging(pfsht_plan* p);
 

@@ -197,10 +197,11 @@ int server_add(pfsht_server* s, pfsht_plan* p, int32_t* id) {
     std::lock_guard<std::mutex> lk(s->mu);
     for (pfsht_plan* q : s->plans)
         if (q == p) return fail(PFSHT_ERR_ARGUMENT, "the plan is registered already");
-    // one coefficient array and one field per direction of the host copies
-    const int64_t staging = 2 * (int64_t)sizeof(double2) *
-                            ((int64_t)(p->L + 1) * (2 * p->L + 1) + p->M) * p->B;
-    const int64_t bytes = p->info.device_bytes + (p->st_alm.p ? 0 : staging);
+    // what it holds, and what it still lacks of one coefficient array and one field per direction of
+    // the host copies
+    const int64_t alm = (int64_t)sizeof(double2) * (p->L + 1) * (2 * p->L + 1) * p->B;
+    const int64_t field = (int64_t)sizeof(double2) * p->M * p->B;
+    const int64_t bytes = plan_bytes(p) + alm * (!p->st_alm.p + !p->st_alm2.p) + field * (!p->st_f.p + !p->st_f2.p);
     if (s->used + bytes > s->budget)
         return fail(PFSHT_ERR_OUT_OF_MEMORY,
                     "registering this plan needs " + std::to_string(bytes) + " bytes of device memory; " +
