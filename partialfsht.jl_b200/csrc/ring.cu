@@ -534,7 +534,8 @@ __device__ __forceinline__ void ring_fwd_walk(const RingTables& t, const RingIte
     }
 }
 
-template <int R, int NB, bool MIX>
+// SPLIT: the item may be one of `size` pieces of its order's degrees, on neighbouring warps of the block
+template <int R, int NB, bool MIX, bool SPLIT>
 __device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut& o,
                                               const RingItem& item, const double2* __restrict__ alm,
                                               double2* __restrict__ out, int b0,
@@ -557,56 +558,72 @@ __device__ __forceinline__ void ring_fwd_item(const RingTables& t, const RingOut
             if (m > 0) ob[jj + o.ld * (o.col_off - m)] = make_double2(gm.x * smir, gm.y * smir);
         }
     };
-    double sc[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int k = lane + 32 * r;
-        sc[r] = k < item.n ? scalbn(t.w ? t.w[item.j0 + k] : 1.0, E[r]) : 0.0;
-    }
-    if (size == 1) {
+    if constexpr (!SPLIT) {
+        // the scale made ring by ring: as an array it costs the batches' forward, whose registers are
+        // full, 3 percent (64 plans: 1.69 against 1.64 ms)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int k = lane + 32 * r;
             if (k >= item.n) continue;
+            const double sc = scalbn(t.w ? t.w[item.j0 + k] : 1.0, E[r]);
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 const double2 tp = accp[r][b].total(), tm = accm[r][b].total();
-                write(k, b, make_double2(tp.x * sc[r], tp.y * sc[r]), make_double2(tm.x * sc[r], tm.y * sc[r]));
+                write(k, b, make_double2(tp.x * sc, tp.y * sc), make_double2(tm.x * sc, tm.y * sc));
             }
         }
-        return;
-    }
-    // the degrees are split over `size` warps of the block: their parts are added in order
-    const int lead = warp - place;
-    auto meet = [&] {
-        if (size == kWarpsPerBlock) asm volatile("bar.sync 1, 128;" ::: "memory");
-        else if (lead == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
-        else asm volatile("bar.sync 2, 64;" ::: "memory");
-    };
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
+    } else {
+        double sc[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const double2 tp = accp[r][b].total(), tm = accm[r][b].total();
-            parts[warp].p[r][lane] = make_double2(tp.x * sc[r], tp.y * sc[r]);
-            parts[warp].m[r][lane] = make_double2(tm.x * sc[r], tm.y * sc[r]);
-        }
-        meet();
-        for (int r = place; r < R; r += size) {
             const int k = lane + 32 * r;
-            if (k < item.n) {
-                double2 gp = parts[lead].p[r][lane], gm = parts[lead].m[r][lane];
-                for (int q = 1; q < size; ++q) {
-                    const double2 up = parts[lead + q].p[r][lane], um = parts[lead + q].m[r][lane];
-                    gp.x += up.x;
-                    gp.y += up.y;
-                    gm.x += um.x;
-                    gm.y += um.y;
-                }
-                write(k, b, gp, gm);
-            }
+            sc[r] = k < item.n ? scalbn(t.w ? t.w[item.j0 + k] : 1.0, E[r]) : 0.0;
         }
-        meet();
+        if (size == 1) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int k = lane + 32 * r;
+                if (k >= item.n) continue;
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    const double2 tp = accp[r][b].total(), tm = accm[r][b].total();
+                    write(k, b, make_double2(tp.x * sc[r], tp.y * sc[r]), make_double2(tm.x * sc[r], tm.y * sc[r]));
+                }
+            }
+            return;
+        }
+        // the degrees are split over `size` warps of the block: their parts are added in order
+        const int lead = warp - place;
+        auto meet = [&] {
+            if (size == kWarpsPerBlock) asm volatile("bar.sync 1, 128;" ::: "memory");
+            else if (lead == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+            else asm volatile("bar.sync 2, 64;" ::: "memory");
+        };
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double2 tp = accp[r][b].total(), tm = accm[r][b].total();
+                parts[warp].p[r][lane] = make_double2(tp.x * sc[r], tp.y * sc[r]);
+                parts[warp].m[r][lane] = make_double2(tm.x * sc[r], tm.y * sc[r]);
+            }
+            meet();
+            for (int r = place; r < R; r += size) {
+                const int k = lane + 32 * r;
+                if (k < item.n) {
+                    double2 gp = parts[lead].p[r][lane], gm = parts[lead].m[r][lane];
+                    for (int q = 1; q < size; ++q) {
+                        const double2 up = parts[lead + q].p[r][lane], um = parts[lead + q].m[r][lane];
+                        gp.x += up.x;
+                        gp.y += up.y;
+                        gm.x += um.x;
+                        gm.y += um.y;
+                    }
+                    write(k, b, gp, gm);
+                }
+            }
+            meet();
+        }
     }
 }
 
@@ -632,7 +649,7 @@ __device__ __forceinline__ void ring_fwd_zero_rest(const RingOut& o, const RingI
     }
 }
 
-template <int RMAX, int NB, bool MIX>
+template <int RMAX, int NB, bool MIX, bool SPLIT = false>
 __device__ __forceinline__ void ring_fwd_body(const RingTables& t, const RingOut& o,
                                               const RingItem& item, const int* __restrict__ jlo,
                                               const int* __restrict__ jhi,
@@ -648,9 +665,9 @@ __device__ __forceinline__ void ring_fwd_body(const RingTables& t, const RingOut
         sub.n = min(32 * RMAX, item.n - base);
         if (sub.ck >= 0) sub.ck += base;
         const int reff = (sub.n + 31) >> 5;
-        if (RMAX >= 4 && reff >= 3) ring_fwd_item<(RMAX >= 4 ? 4 : 1), NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
-        else if (RMAX >= 2 && reff == 2) ring_fwd_item<(RMAX >= 2 ? 2 : 1), NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
-        else ring_fwd_item<1, NB, MIX>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
+        if (RMAX >= 4 && reff >= 3) ring_fwd_item<(RMAX >= 4 ? 4 : 1), NB, MIX, SPLIT>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
+        else if (RMAX >= 2 && reff == 2) ring_fwd_item<(RMAX >= 2 ? 2 : 1), NB, MIX, SPLIT>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
+        else ring_fwd_item<1, NB, MIX, SPLIT>(t, o, sub, alm, out, b0, sm, warp, lane, parts, size, place);
     }
 }
 
@@ -677,8 +694,8 @@ ring_fwd_split_kernel(RingTables t, RingOut o, const RingItem* __restrict__ bloc
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const RingItem item = blocks[blockIdx.x * kWarpsPerBlock + warp];
     if (item.n == 0) return;
-    ring_fwd_body<RMAX, NB, MIX>(t, o, item, jlo, jhi, alm, out, b0, sm[warp], warp, lane, parts,
-                                 item.pad_ & 0xff, item.pad_ >> 8);
+    ring_fwd_body<RMAX, NB, MIX, true>(t, o, item, jlo, jhi, alm, out, b0, sm[warp], warp, lane, parts,
+                                       item.pad_ & 0xff, item.pad_ >> 8);
 }
 
 // ---------------------------------------------------------------------------------------
