@@ -378,6 +378,11 @@ int tma_timeouts(int* out);
 // window for kernel width w, and the two passes
 int mma_tile_cols(int w);
 int mma_max_advance();
+// kernel width from which interpolation runs on the matrix instruction too: below it the
+// thread-per-point kernels are as fast or faster (lmax 1024, 511,063 points: 37 us against 44 at
+// w = 9, 50 against 52 at w = 10, but 63 against 54 at w = 11 and 140 against 84 at w = 16; 6 to 20
+// points per 100 grid cells: 33-37 against 27-31 at w = 11)
+constexpr int kMmaInterpWidth = 11;
 struct MmaGroup {
     int first, n;  // sorted points [first, first + n), n <= 8
     int strip;     // strip of the first of them

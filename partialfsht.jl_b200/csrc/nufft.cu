@@ -269,11 +269,6 @@ static int interp_point_order(const NufftGrid& g, NufftDev& d, const double2* pt
     return 0;
 }
 
-// kernel width from which interpolation runs on the matrix instruction too: below it the
-// thread-per-point kernels are as fast or faster (lmax 1024, 511,063 points: 37 us against 44 at
-// w = 9, 50 against 52 at w = 10, but 63 against 54 at w = 11 and 140 against 84 at w = 16; 6 to 20
-// points per 100 grid cells: 33-37 against 27-31 at w = 11)
-constexpr int kMmaInterpWidth = 11;
 // points of an item and its most strips. Fewer points or strips make more and shorter items, which
 // pay for the edges of their windows but fill the GPU where there are few points: with strips
 // unbounded, spreading 10,000 points at lmax 1024 took 40 us, at most 8 strips 20, at most 4 22;

@@ -203,7 +203,7 @@ __device__ __forceinline__ double weight(unsigned a) {
 }
 
 template <int W>
-__global__ void __launch_bounds__(kWarps * 32, W <= 9 ? 6 : W <= 13 ? 5 : 3)
+__global__ void __launch_bounds__(kWarps * 32, W <= 13 ? 5 : 3)
 interp_mma_kernel(const double2* __restrict__ off, const int2* __restrict__ meta,
                   const int4* __restrict__ items, int nitems, const double2* __restrict__ U,
                   int nrows, int nf2, int row_wrap, int64_t M, double2* __restrict__ f) {
@@ -454,12 +454,17 @@ int set_smem(K kernel, size_t bytes) {
 
 template <int W>
 int launch_interp_mma(const NufftGrid& g, NufftDev& d, double2* f, int B, cudaStream_t s) {
-    const size_t smem = kWarps * sizeof(Stage<W>);
-    PF_TRY(set_smem(interp_mma_kernel<W>, smem));
-    interp_mma_kernel<W><<<dim3((g.nitems + kWarps - 1) / kWarps, B), kWarps * 32, smem, s>>>(
-        d.soff.as<double2>(), d.smeta.as<int2>(), d.items.as<int4>(), g.nitems, d.U.as<double2>(), g.nrows, g.nf2,
-        g.row_wrap, g.M, f);
-    return check_launch("interp_mma_kernel");
+    if constexpr (W < kMmaInterpWidth) {
+        set_error("interpolation of this width does not run on the matrix instruction");
+        return 7;
+    } else {
+        const size_t smem = kWarps * sizeof(Stage<W>);
+        PF_TRY(set_smem(interp_mma_kernel<W>, smem));
+        interp_mma_kernel<W><<<dim3((g.nitems + kWarps - 1) / kWarps, B), kWarps * 32, smem, s>>>(
+            d.soff.as<double2>(), d.smeta.as<int2>(), d.items.as<int4>(), g.nitems, d.U.as<double2>(), g.nrows, g.nf2,
+            g.row_wrap, g.M, f);
+        return check_launch("interp_mma_kernel");
+    }
 }
 
 template <int W>

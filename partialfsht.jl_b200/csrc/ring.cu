@@ -683,19 +683,20 @@ ring_fwd_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int
     ring_fwd_body<RMAX, NB, MIX>(t, o, items[it], jlo, jhi, alm, out, b0, sm[warp], warp, lane);
 }
 
-// the same with the items in blocks, whose warps may share an item's degrees
-template <int RMAX, int NB, bool MIX>
+// the same with the items in blocks, whose warps may share an item's degrees (FP64 tables: the mixed
+// form's stretched plans have them for the forward too)
+template <int RMAX, int NB>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, RMAX >= 4 ? 3 : NB == 1 ? 5 : NB == 2 ? 4 : 3)
 ring_fwd_split_kernel(RingTables t, RingOut o, const RingItem* __restrict__ blocks,
                       const int* __restrict__ jlo, const int* __restrict__ jhi,
                       const double2* __restrict__ alm, double2* __restrict__ out, int b0) {
-    __shared__ FwdSmem<NB, MIX> sm[kWarpsPerBlock];
+    __shared__ FwdSmem<NB, false> sm[kWarpsPerBlock];
     __shared__ FwdPart parts[kWarpsPerBlock];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const RingItem item = blocks[blockIdx.x * kWarpsPerBlock + warp];
     if (item.n == 0) return;
-    ring_fwd_body<RMAX, NB, MIX, true>(t, o, item, jlo, jhi, alm, out, b0, sm[warp], warp, lane, parts,
-                                       item.pad_ & 0xff, item.pad_ >> 8);
+    ring_fwd_body<RMAX, NB, false, true>(t, o, item, jlo, jhi, alm, out, b0, sm[warp], warp, lane, parts,
+                                         item.pad_ & 0xff, item.pad_ >> 8);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1232,11 +1233,13 @@ static int launch_fwd(const RingTables& t, const RingOut& o, const RingItems& v,
                       double2* out, int b0, cudaStream_t s) {
     const RingItem* items = v.items;
     const int nitems = v.nitems, *jlo = v.jlo, *jhi = v.jhi;
-    if (v.blocks) {
-        if (v.nblocks <= 0) return 0;
-        ring_fwd_split_kernel<RMAX, NB, MIX><<<v.nblocks, kWarpsPerBlock * 32, 0, s>>>(t, o, v.blocks, jlo, jhi,
-                                                                                       alm, out, b0);
-        return check_launch("ring_fwd_split_kernel");
+    if constexpr (!MIX) {
+        if (v.blocks) {
+            if (v.nblocks <= 0) return 0;
+            ring_fwd_split_kernel<RMAX, NB><<<v.nblocks, kWarpsPerBlock * 32, 0, s>>>(t, o, v.blocks, jlo, jhi, alm,
+                                                                                      out, b0);
+            return check_launch("ring_fwd_split_kernel");
+        }
     }
     const int grid = (nitems + kWarpsPerBlock - 1) / kWarpsPerBlock;
     ring_fwd_kernel<RMAX, NB, MIX><<<grid, kWarpsPerBlock * 32, 0, s>>>(t, o, items, nitems, jlo, jhi,
