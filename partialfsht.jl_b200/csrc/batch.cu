@@ -59,7 +59,6 @@ struct pfsht_batch {
     pf::DevBuf stf;      // double2*[n]: each plan's field buffer
     pf::DevBuf chunks;   // FChunk[nchunks]
     int nchunks = 0;
-    std::unique_ptr<pf::RingSegments[]> adj_seg;  // [n], the adjoint items' saved states where not the plan's
     cudaStream_t main = nullptr;
     std::vector<cudaStream_t> side;
     cudaEvent_t fork = nullptr, done = nullptr;
@@ -211,9 +210,6 @@ int batch_create(pfsht_plan* const* plans, int n, int nstreams, pfsht_batch** ou
     std::vector<double2*> stf(n);
     std::vector<FChunk> chunks;
     std::vector<RingBatchPlan> fw(n), ad(n);
-    const std::vector<int> degrees = batch_adjoint_degrees(plans, n);
-    b->adj_seg.reset(new RingSegments[n]);
-    std::vector<std::vector<RingItem>> adj(n);
     for (int i = 0; i < n; ++i) {
         pfsht_plan* p = plans[i];
         const size_t nf = sizeof(double2) * (size_t)p->M * p->B;
@@ -222,7 +218,7 @@ int batch_create(pfsht_plan* const* plans, int n, int nstreams, pfsht_batch** ou
         if (!p->H.p) PF_TRY(p->H.alloc(sizeof(double2) * (size_t)p->ro_cols.bstride * p->B));
         stf[i] = p->st_f.as<double2>();
         RingSlot& s = slots[i];
-        if (!p->spin) PF_TRY(batch_adjoint_items(p, degrees[i], s.t, b->adj_seg[i], adj[i], b->main));
+        s.t = p->rt;
         s.tf = p->rt_fwd;
         s.o = p->ro_cols;
         s.jlo = p->adj_items.view.jlo;
@@ -234,7 +230,7 @@ int batch_create(pfsht_plan* const* plans, int n, int nstreams, pfsht_batch** ou
         // scalar recurrence)
         static const std::vector<RingItem> kNone;
         fw[i] = RingBatchPlan{p->spin ? &kNone : &p->fwd_items.host, p->B, p->fwd_items.view.rmax, p->rt_fwd.mix};
-        ad[i] = RingBatchPlan{&adj[i], p->B, p->adj_items.view.rmax, p->rt.mix};
+        ad[i] = RingBatchPlan{p->spin ? &kNone : &p->adj_items.host, p->B, p->adj_items.view.rmax, p->rt.mix};
         const int64_t tot = p->M * p->B;
         for (int64_t o = 0; o < tot; o += kFChunk) chunks.push_back(FChunk{i, o, std::min(kFChunk, tot - o)});
     }

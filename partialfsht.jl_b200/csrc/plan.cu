@@ -216,23 +216,29 @@ void fill_info(pfsht_plan* p) {
     }
 }
 
+// Adjoint items: tiles of 32 * R rings whose sums add atomically when an order spans several;
+// with the deterministic option, all retained rings of an order in one item when no order retains
+// more than four tiles (the warp walks them tile after tile and adds each tile's sums to the
+// previous ones in order: a pass without atomics, measured ~8% slower at lmax 2048); each order split into degree segments of about seg_degrees when the
+// unsplit items would give fewer than ~8 warps per resident warp slot (12 per SM at the
+// adjoint's register count). The saved recurrence state is bounded by 512 MiB; past that, or
+// with seg_degrees < 0, the items stay whole.
 // Degree-segment length of the adjoint's items, from a model of the ring pass: an item of d
 // degrees whose lanes hold R rings costs d (6 R + 4) (the recurrence and the four sums per ring,
 // the transpose-reduce per degree) plus 400 for its start (seed or saved state, ring data, first
-// coefficients: about 60 degrees' work); items are dealt heaviest first to the warp slots (11 per SM:
-// fitted to the lengths that ran fastest and not the 16 resident warps, which picked slower ones,
-// lmax 2048 252 against 249 us), and the length of 64 q degrees, q from `shortest` to 8, with the
-// shortest schedule wins. Adjoint ring pass against fixed
+// coefficients: about 60 degrees' work); items are dealt heaviest first to the resident warp
+// slots (shared by the transforms of an apply), and the segment length of 64 q degrees (q = 1..8)
+// with the shortest schedule wins. Adjoint ring pass against fixed
 // lengths, one transform at lmax 256 / 1024 / 2048: 16.5 / 64.5 / 263.5 us as picked (64 / 128 / 448
 // degrees), 30.5 / 72.3 / 271.1 at 256 degrees; 128 degrees, the shortest length before, took 20.9 at
 // lmax 256. Four transforms at lmax 1024: 213.1 as picked, 220.2 at 128. The model is not exact: its
 // picks were up to 10 percent off the best length (four transforms at lmax 384: 42.8, 38.6 at 192).
 static int choose_segment_degrees(const std::vector<int>& jlo, const std::vector<int>& jhi, int L,
-                                  int mmax, int tile, int rmax, int slots, int shortest) {
+                                  int mmax, int tile, int rmax, int slots) {
     std::vector<double> cost;
     double best = 0.0;
     int best_q = 0;
-    for (int q = shortest; q <= 8; ++q) {
+    for (int q = 1; q <= 8; ++q) {
         cost.clear();
         for (int m = 0; m <= std::min(mmax, L); ++m) {
             if (jhi[m] < jlo[m]) continue;
@@ -269,50 +275,29 @@ static int choose_segment_degrees(const std::vector<int>& jlo, const std::vector
     return 64 * best_q;
 }
 
-// Adjoint items: tiles of 32 * R rings whose sums add atomically when an order spans several;
-// with the deterministic option, all retained rings of an order in one item when no order retains
-// more than four tiles (the warp walks them tile after tile and adds each tile's sums to the
-// previous ones in order: a pass without atomics, measured ~8% slower at lmax 2048); each order split
-// into degree segments of about adjoint_degrees when the unsplit items would give fewer than ~8 warps
-// per slot of 12 per SM. The saved recurrence state is bounded by 512 MiB; past that, or
-// with seg_degrees < 0, the items stay whole.
-constexpr int64_t kMaxSavedState = (int64_t)512 << 20;
-int adjoint_rings(const pfsht_plan* p) { return p->R > 0 ? p->R : 4; }
-int adjoint_slots(const pfsht_plan* p) {
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
-    return sms * 11;
-}
-int adjoint_tile(const pfsht_plan* p, const std::vector<int>& jlo, const std::vector<int>& jhi, int mmax) {
-    const int rmax = adjoint_rings(p);
-    int maxret = 0;
-    for (int m = 0; m <= std::min(mmax, p->L); ++m) maxret = std::max(maxret, jhi[m] - jlo[m] + 1);
-    return p->deterministic && maxret <= 4 * 32 * rmax ? std::max(maxret, 1) : 32 * rmax;
-}
-
-// An apply of the plan alone shares the slots among its transforms and may cut down to 64 degrees. In a
-// batch the other plans' items fill the GPU, and more, shorter items only add starts and atomic sums: each
-// transform counts as the only one, from 128 degrees. Adjoint of 64 plans 6.36 ms, with 64 degrees
-// allowed 6.64, with the slots shared 6.52, with the plans' own lengths 6.55.
-int adjoint_degrees(const pfsht_plan* p, const std::vector<int>& jlo, const std::vector<int>& jhi, int mmax,
-                    bool in_batch) {
-    if (p->seg_degrees != 0) return p->seg_degrees;
-    const int rmax = adjoint_rings(p), tile = adjoint_tile(p, jlo, jhi, mmax), slots = adjoint_slots(p);
-    if (make_ring_items(jlo, jhi, p->L, mmax, tile).size() >= (size_t)slots / 11 * 12 * 8) return -1;
-    return choose_segment_degrees(jlo, jhi, p->L, mmax, tile, rmax, in_batch ? slots : std::max(1, slots / p->B),
-                                  in_batch ? 2 : 1);
-}
-
 int build_adjoint_items(pfsht_plan* p, const std::vector<int>& jlo, const std::vector<int>& jhi,
                         int mmax, cudaStream_t s) {
-    p->adj_degrees = adjoint_degrees(p, jlo, jhi, mmax, false);
-    if (p->adj_degrees > 0) {
-        PF_TRY(build_ring_segments(p->rt, jlo, jhi, p->L, mmax, p->adj_degrees, kMaxSavedState, p->adj_seg, s));
+    const int L = p->L;
+    const int rmax = p->R > 0 ? p->R : 4;
+    int maxret = 0;
+    for (int m = 0; m <= std::min(mmax, L); ++m) maxret = std::max(maxret, jhi[m] - jlo[m] + 1);
+    const int tile = p->deterministic && maxret <= 4 * 32 * rmax ? std::max(maxret, 1) : 32 * rmax;
+    int seg = p->seg_degrees;
+    if (seg == 0) {
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+        const size_t whole = make_ring_items(jlo, jhi, L, mmax, tile).size();
+        const int slots = std::max(1, sms * 11 / p->B);
+        seg = whole >= (size_t)sms * 12 * 8 ? -1
+                                            : choose_segment_degrees(jlo, jhi, L, mmax, tile, rmax, slots);
+    }
+    if (seg > 0) {
+        PF_TRY(build_ring_segments(p->rt, jlo, jhi, L, mmax, seg, (int64_t)512 << 20, p->adj_seg, s));
         p->rt.ck_p = p->adj_seg.ck_p.as<double2>();
         p->rt.ck_E = p->adj_seg.ck_E.as<int>();
     }
-    return build_ring_items(jlo, jhi, p->L, mmax, adjoint_rings(p), p->adj_items, s,
-                            p->adj_seg.seg_degrees > 0 ? &p->adj_seg : nullptr, adjoint_tile(p, jlo, jhi, mmax));
+    return build_ring_items(jlo, jhi, L, mmax, rmax, p->adj_items, s,
+                            p->adj_seg.seg_degrees > 0 ? &p->adj_seg : nullptr, tile);
 }
 
 // The Direct leaf's FP64 scalar applies take the points' phases inside their ring passes (eight rings
@@ -928,59 +913,6 @@ int64_t plan_bytes(const pfsht_plan* p) {
         bytes += (int64_t)b->bytes;
     for (const auto& c : p->boxes) bytes += plan_bytes(c.get());
     return bytes;
-}
-
-// retained rings of the plan's orders
-static void plan_rings(const pfsht_plan* p, std::vector<int>& jlo, std::vector<int>& jhi, int& mmax) {
-    if (p->kind == kDirect) {
-        jlo.assign(p->L + 1, 0);
-        jhi.assign(p->L + 1, (int)p->M - 1);
-        mmax = p->L;
-    } else {
-        jlo = p->leaf.jlo;
-        jhi = p->leaf.jhi;
-        mmax = p->leaf.mmax;
-    }
-}
-
-std::vector<int> batch_adjoint_degrees(pfsht_plan* const* plans, int n) {
-    // the plans' own lengths while the batch is little more than one plan: adjoint of the first 1, 2, 4, 8
-    // of 64 plans (0.9, 1.0, 1.8, 3.5 whole items per slot) with their own lengths 0.384, 0.393, 0.511,
-    // 0.799 ms, with the batch's 0.391, 0.404, 0.521, 0.783
-    std::vector<int> degrees(n, 0);
-    double whole = 0.0;
-#pragma omp parallel for schedule(dynamic, 1) reduction(+ : whole)
-    for (int i = 0; i < n; ++i) {
-        const pfsht_plan* p = plans[i];
-        if (p->spin) continue;  // its adjoint is not merged
-        std::vector<int> jlo, jhi;
-        int mmax;
-        plan_rings(p, jlo, jhi, mmax);
-        whole += (double)p->B * make_ring_items(jlo, jhi, p->L, mmax, adjoint_tile(p, jlo, jhi, mmax)).size();
-        degrees[i] = adjoint_degrees(p, jlo, jhi, mmax, true);
-    }
-    if (whole < 2.5 * adjoint_slots(plans[0]))
-        for (int i = 0; i < n; ++i) degrees[i] = plans[i]->adj_degrees;
-    return degrees;
-}
-
-int batch_adjoint_items(const pfsht_plan* p, int degrees, RingTables& t, RingSegments& seg,
-                        std::vector<RingItem>& items, cudaStream_t s) {
-    t = p->rt;
-    if (degrees == p->adj_degrees) {
-        items = p->adj_items.host;
-        return 0;
-    }
-    std::vector<int> jlo, jhi;
-    int mmax;
-    plan_rings(p, jlo, jhi, mmax);
-    if (degrees > 0) {
-        PF_TRY(build_ring_segments(t, jlo, jhi, p->L, mmax, degrees, kMaxSavedState, seg, s));
-        t.ck_p = seg.ck_p.as<double2>();
-        t.ck_E = seg.ck_E.as<int>();
-    }
-    items = make_ring_items(jlo, jhi, p->L, mmax, adjoint_tile(p, jlo, jhi, mmax), seg.seg_degrees > 0 ? &seg : nullptr);
-    return 0;
 }
 
 int plan_forward_after_ring(pfsht_plan* p, double2* f, cudaStream_t s, bool in_batch) {

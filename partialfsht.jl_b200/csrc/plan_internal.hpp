@@ -30,7 +30,6 @@ struct pfsht_plan {
     RingSegments fwd_seg;  // degree segments of the forward's blocks
     RingSegments adj_seg;  // degree segments of the adjoint items
     int seg_degrees = 0;   // requested segment length (0 = auto, < 0 = none)
-    int adj_degrees = 0;   // the adjoint's segment length for applies of this plan alone
     RingTables rt;
     // the forward ring pass's tables: rt itself, except in the mixed form, whose forward runs the
     // FP64 pass (FP32 accumulation saves nothing there: each ring value's conversion costs as
@@ -140,11 +139,6 @@ int plan_host_enqueue(pfsht_plan* p, const void* in, void* out, bool fwd, cudaSt
                       bool order_on_s = true, bool zero_async = false);
 // wait for the plan's asynchronous padding zeroing, if one is running
 void plan_host_wait(pfsht_plan* p);
-// The scalar plans' adjoint ring items in a batch: the segment lengths (host work only), and a plan's
-// items with the tables that hold their saved states (`seg`, which the batch keeps)
-std::vector<int> batch_adjoint_degrees(pfsht_plan* const* plans, int n);
-int batch_adjoint_items(const pfsht_plan* p, int degrees, RingTables& t, RingSegments& seg,
-                        std::vector<RingItem>& items, cudaStream_t s);
 int64_t plan_bytes(const pfsht_plan* p);  // device memory the plan holds now
 // allocate the plan's staging buffers for host-buffer applies
 int plan_host_staging(pfsht_plan* p);
