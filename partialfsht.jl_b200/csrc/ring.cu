@@ -1558,7 +1558,7 @@ static int adj_batch_shape(const RingSlot* slots, const RingBatchGroup& g, void*
 
 // ---------------------------------------------------------------------------------------
 // one persistent launch per direction for the ring passes of many plans: each warp pulls the next
-// item (any plan, any tile shape; all items heaviest first) from a counter in device memory until
+// item (any plan, any tile shape; heaviest first by classes) from a counter in device memory until
 // none is left, and the item's shape code (RingItem::pad_) selects the pass it runs. A block
 // holds one staging area per warp, sized for the largest shape, so warps of one block may run
 // different shapes. No warp waits for another.
@@ -1662,7 +1662,21 @@ int build_ring_merged(const std::vector<RingBatchPlan>& plans, bool adjoint, Rin
             all.push_back({cost, b});
         }
     }
-    std::stable_sort(all.begin(), all.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+    // Heaviest first, so that the last items to end are short ones, but only by classes of a factor of four,
+    // and plan by plan within a class: neighbouring warps then read the same plan's columns and
+    // coefficients. Strictly by cost the plans alternate, the more so the more items have nearly the same
+    // cost: 64 plans (adjoint / forward) 6.57 / 3.84 ms, in classes of 1.2 6.19 / 3.65, of 2 6.02 / 3.59, of 4
+    // 5.96 / 3.57, plan by plan alone 5.93 / 3.60; 16 plans with a few large ones 1.57 / 1.18, 1.57 / 1.18,
+    // 1.55 / 1.18, 1.51 / 1.18, 1.51 / 1.24
+    auto cost_class = [](int64_t cost) {
+        int k = 0;
+        for (; cost >= 4; cost /= 4) ++k;
+        return k;
+    };
+    std::stable_sort(all.begin(), all.end(), [&](const auto& a, const auto& b) {
+        const int ka = cost_class(a.first), kb = cost_class(b.first);
+        return ka != kb ? ka > kb : a.second.slot < b.second.slot;
+    });
     std::vector<BatchItem> items(all.size());
     for (size_t i = 0; i < all.size(); ++i) items[i] = all[i].second;
     mg.nitems = (int)items.size();
