@@ -216,12 +216,16 @@ def hbm_peak():
     return 6650.0, "6650 GB/s (of fallback: MEASURED_PEAKS.json absent)"
 
 
-def load_traffic():
+def load_traffic(info, B=1):
+    """The stored ncu bytes per launch of each stage, for the workload they were captured at."""
     p = os.path.join(ROOT, "profiles", "traffic_per_launch.json")
     try:
-        return json.load(open(p))
+        stored = json.load(open(p))
     except (OSError, ValueError):
         return {}
+    here = dict(info, ntrans=B)
+    same = all(here.get(k, v if k == "precision" else None) == v for k, v in stored["workload"].items())
+    return stored["bytes"] if same else {}
 
 
 def stage_work(info, stage, B=1):
@@ -255,7 +259,7 @@ def stage_work(info, stage, B=1):
 def stage_rooflines(info, stages, fp64_peak, hbm, B=1):
     """Per stage of our own kernels: time per launch, algorithmic FP64 rate and bytes rate against
     the measured peaks, and the DRAM rate from the ncu traffic per launch where one is recorded."""
-    traffic = load_traffic()
+    traffic = load_traffic(info, B)
     out = {}
     for k, (tot, n) in stages.items():
         if k.startswith("fft_"):
@@ -886,7 +890,7 @@ def run_b200(args, world, rank, local):
     dom_ms = ours[dom][0] / ours[dom][1]
     flops, byts = stage_work(info, dom, B)
     hbm, hbm_source = hbm_peak()
-    traffic = load_traffic().get(dom)
+    traffic = load_traffic(info, B).get(dom)
     if flops / (fp64_peak * 1e12) >= byts / (hbm * 1e9):
         achieved = flops / (dom_ms * 1e-3) / 1e12
         roof = {"bound": "fp64", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
