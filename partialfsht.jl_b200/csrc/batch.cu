@@ -4,7 +4,7 @@
 // One direction of a batch is one CUDA graph, captured on first use and replayed with a single
 // cudaGraphLaunch:
 //   forward : pointer table -> ring passes of all scalar plans (one persistent launch: warps
-//             pull the items of every plan and tile shape, heaviest first, from a counter) ->
+//             pull the items of every plan and tile shape, heaviest classes first, from a counter) ->
 //             per plan, on one of several streams: the
 //             spin ring pass of a spin plan, FFT along Theta and NUFFT type 2 into the plan's
 //             own field buffer -> one copy kernel into the callers' fields

@@ -171,7 +171,7 @@ struct RingBatchPlan {
     const std::vector<RingItem>* items;
     int B, rmax, mix;
 };
-// all plans' items of one direction in one persistent launch (every tile shape, heaviest first)
+// all plans' items of one direction in one persistent launch (every tile shape, by classes of cost, build_ring_merged)
 struct RingMerged {
     DevBuf items;    // BatchItem[nitems], it.pad_ = shape code
     DevBuf counter;  // next item to pull

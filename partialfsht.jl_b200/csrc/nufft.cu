@@ -1720,7 +1720,7 @@ static int launch_interp(const NufftGrid& g, NufftDev& d, double2* f, int B, cud
     const size_t smem = sizeof(cx<T>) * (size_t)tile_elems;
     PF_TRY(allow_smem(interp_kernel<W, T>, smem));
     // a transform per row of blocks; in a batch, whose other plans fill the GPU, a block takes all of its
-    // group's transforms (64 plans: 3.88 against 3.98 ms a forward)
+    // group's transforms (64 plans: 3.58 against 3.70 ms a forward)
     interp_kernel<W, T><<<dim3(g.nisb, g.in_batch ? 1 : B), 128, smem, s>>>(
         d.ipts.as<double2>(), d.iperm.as<int>(), d.binstart.as<int>(), d.iorder.as<int>(), g.nbc,
         g.igroup, g.nsbc, g.bin_rows, g.bin_cols, g.M, d.U.as<cx<T>>(), g.nrows, g.nf2,

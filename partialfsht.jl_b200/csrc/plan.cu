@@ -219,16 +219,17 @@ void fill_info(pfsht_plan* p) {
 // Adjoint items: tiles of 32 * R rings whose sums add atomically when an order spans several;
 // with the deterministic option, all retained rings of an order in one item when no order retains
 // more than four tiles (the warp walks them tile after tile and adds each tile's sums to the
-// previous ones in order: a pass without atomics, measured ~8% slower at lmax 2048); each order split into degree segments of about seg_degrees when the
-// unsplit items would give fewer than ~8 warps per resident warp slot (12 per SM at the
-// adjoint's register count). The saved recurrence state is bounded by 512 MiB; past that, or
+// previous ones in order: a pass without atomics, measured ~8% slower at lmax 2048); each order split
+// into degree segments of about seg_degrees when the unsplit items would give fewer than ~8 warps
+// for each of 12 slots per SM. The saved recurrence state is bounded by 512 MiB; past that, or
 // with seg_degrees < 0, the items stay whole.
 // Degree-segment length of the adjoint's items, from a model of the ring pass: an item of d
 // degrees whose lanes hold R rings costs d (6 R + 4) (the recurrence and the four sums per ring,
 // the transpose-reduce per degree) plus 400 for its start (seed or saved state, ring data, first
-// coefficients: about 60 degrees' work); items are dealt heaviest first to the resident warp
-// slots (shared by the transforms of an apply), and the segment length of 64 q degrees (q = 1..8)
-// with the shortest schedule wins. Adjoint ring pass against fixed
+// coefficients: about 60 degrees' work); items are dealt heaviest first to 11 warp slots per SM
+// (fitted to the lengths that ran fastest; the 16 resident warps picked slower ones, lmax 2048 252
+// against 249 us), shared by the transforms of an apply, and the segment length of 64 q degrees
+// (q = 1..8) with the shortest schedule wins. Adjoint ring pass against fixed
 // lengths, one transform at lmax 256 / 1024 / 2048: 16.5 / 64.5 / 263.5 us as picked (64 / 128 / 448
 // degrees), 30.5 / 72.3 / 271.1 at 256 degrees; 128 degrees, the shortest length before, took 20.9 at
 // lmax 256. Four transforms at lmax 1024: 213.1 as picked, 220.2 at 128. The model is not exact: its

@@ -684,7 +684,10 @@ ring_fwd_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int
 }
 
 // the same with the items in blocks, whose warps may share an item's degrees (FP64 tables: the mixed
-// form's stretched plans have them for the forward too)
+// form's stretched plans have them for the forward too). Blocks per SM: with one less the shapes of two
+// rings a lane spill nothing (16 to 48 bytes as they are), and the passes take, lmax 1024 / 2048, one
+// transform 45.3 / 189 us instead of 44.0 / 177, two 70.6 / 318 instead of 66.4 / 305, four 129.5 / 596
+// instead of 116 / 556 (lmax 256, four transforms: 19.3 instead of 21.8)
 template <int RMAX, int NB>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, RMAX >= 4 ? 3 : NB == 1 ? 5 : NB == 2 ? 4 : 3)
 ring_fwd_split_kernel(RingTables t, RingOut o, const RingItem* __restrict__ blocks,
@@ -1180,10 +1183,12 @@ __device__ __forceinline__ void ring_adj_body(const RingTables& t, const RingOut
 
 // Up to four rings a lane: 16 one-warp blocks per SM, i.e. 128 registers instead of the 164 that the
 // compiler takes for itself in FP64 (12 blocks); the FP32 sums fit without (126), but take more when
-// one block is asked for (lmax 2048, both directions: 764 against 727 us). The pass is bound by shared-memory wavefronts (76 percent of
-// their peak, FP64 55) and by the latency that so few warps leave open: at lmax 1024 / 2048, 64.5 to
-// 62.3 and 263.5 to 249.2 us, four transforms at 1024 213 to 202. Sums over the lanes without shared
-// memory (butterflies of the lanes, at the same registers) took 68.5 and 288 us, 18 blocks (spills) 261.
+// one block is asked for (lmax 2048, both directions: 764 against 727 us). At lmax 1024 / 2048, 64.5 to
+// 62.3 and 263.5 to 249.2 us, four transforms at 1024 213 to 202. No unit is full: the shared-memory unit is
+// busy 84 percent, FP64 58, issue slots 48; and the FP32 sums, with half the shared-memory wavefronts and a
+// third of the FP64 work, take 96 percent of the time. What is left is the dependent chain of each degree at
+// 15 warps. Sums over the lanes without shared memory (butterflies of the lanes, at the same registers)
+// took 68.5 and 288 us, 18 blocks (spills) 261.
 template <int RMAX, int NB, bool MIX, bool PHASE>
 __global__ void __launch_bounds__(kAdjWarps * 32, RMAX <= 4 ? 16 : 8)
 ring_adj_kernel(RingTables t, RingOut o, const RingItem* __restrict__ items, int nitems,

@@ -9,12 +9,14 @@
 // freezes the updates, exactly where the reference's loop breaks. The host keeps one iteration in
 // flight: it launches iteration i, then waits for the state copied out after iteration i - 1, and
 // stops when that says done (the iteration in flight is then a frozen no-op). The launches go
-// straight to the caller's stream: an iteration's kernels take longer than their launches (109
-// against about 60 us at lmax 256), while capturing them as a graph for each solve, with the
-// workspace allocated and freed each time, cost 4 ms and more (8 iterations at lmax 384: 5.9 ms
-// against 1.1). Dot products reduce in a fixed order (per-block partials, then one block); the adjoint apply inside an iteration adds floating-point atomically (ring tiles of one
-// order, spread rows shared by neighbouring bins), so two solves agree to round-off, not bit for
-// bit.
+// straight to the caller's stream. An iteration's kernels mostly take longer than their launches (109
+// against about 60 us at lmax 256), while capturing them as a graph for each solve, with the workspace
+// allocated and freed each time, cost 4 ms and more (8 iterations at lmax 384: 5.9 ms against 1.1). Over
+// 400 iterations, us each, graph against launches: cap at lmax 64 89-102 / 94, 128 101-110 / 100, 256 137-162
+// / 112; Direct with 400 points 85-116 / 61; two boxes 240-248 / 158, three 311-326 / 149, four 445-452 /
+// 252. Dot products reduce in a fixed order (per-block partials, then one block); the adjoint apply inside
+// an iteration adds floating-point atomically (ring tiles of one order, spread rows shared by
+// neighbouring bins), so two solves agree to round-off, not bit for bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
