@@ -113,7 +113,7 @@ int record(pfsht_batch* b, bool fwd) {
             if (p->spin)
                 PF_TRY(spin_ring_forward_ptr(p->spt.t, p->ro_cols, p->fwd_items.view, ptrs, i,
                                              p->H.as<double2>(), p->B, s));
-            PF_TRY(plan_forward_after_ring(p, p->st_f.as<double2>(), s, true));
+            PF_TRY(plan_forward_after_ring(p, p->st_f.as<double2>(), s));
         } else if (p->spin) {
             PF_TRY(plan_adjoint_before_ring(p, p->st_f.as<double2>(), s));
             PF_TRY(alm_prepare_ptr(ptrs, i, p->L, p->B, nullptr, 0, s));

@@ -336,7 +336,6 @@ struct NufftGrid {
     int mma = 0, mma_interp = 0;
     int blk_cols = 1, item_rows = 1 << 20, nitems = 0;
     int cols = 0;              // the column stages run as one kernel each way (nufft_cols.cu)
-    int in_batch = 0;          // 1: the launches are a batch's, beside those of other plans
     int interp_pipe = 1;       // one-transform interpolation copies the next group's tile ahead
 };
 

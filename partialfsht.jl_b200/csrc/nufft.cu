@@ -948,7 +948,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 5 : 4)
 interp_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
               const int* __restrict__ binstart, const int* __restrict__ iorder, int nbc, int G,
               int nsbc, int BR, int BC, int64_t M, const cx<T>* __restrict__ U, int nrows,
-              int nf2, int row_wrap, int B, double2* __restrict__ f) {
+              int nf2, int row_wrap, double2* __restrict__ f) {
     extern __shared__ __align__(16) unsigned char interp_smem[];
     cx<T>* tile = reinterpret_cast<cx<T>*>(interp_smem);
     // a group of G consecutive bins of one bin row: their points are contiguous in bin order
@@ -963,7 +963,8 @@ interp_kernel(const double2* __restrict__ pts, const int* __restrict__ perm,
     // tile rows an odd number of elements apart: a tap's bank class then depends on its row as
     // well as its column, which evens out the classes the points are dealt over
     const int TS = tg.TC | 1;
-    for (int b = blockIdx.y; b < B; b += gridDim.y) {  // transforms
+    {
+        const int b = blockIdx.y;  // transform
         const cx<T>* ub = U + (int64_t)nrows * nf2 * b;
         if (tg.TC <= 32) {
             if (ln < tg.TC) {
@@ -1719,12 +1720,10 @@ static int launch_interp(const NufftGrid& g, NufftDev& d, double2* f, int B, cud
     }
     const size_t smem = sizeof(cx<T>) * (size_t)tile_elems;
     PF_TRY(allow_smem(interp_kernel<W, T>, smem));
-    // a transform per row of blocks; in a batch, whose other plans fill the GPU, a block takes all of its
-    // group's transforms (64 plans: 3.58 against 3.70 ms a forward)
-    interp_kernel<W, T><<<dim3(g.nisb, g.in_batch ? 1 : B), 128, smem, s>>>(
+    interp_kernel<W, T><<<dim3(g.nisb, B), 128, smem, s>>>(
         d.ipts.as<double2>(), d.iperm.as<int>(), d.binstart.as<int>(), d.iorder.as<int>(), g.nbc,
         g.igroup, g.nsbc, g.bin_rows, g.bin_cols, g.M, d.U.as<cx<T>>(), g.nrows, g.nf2,
-        g.row_wrap, B, f);
+        g.row_wrap, f);
     return check_launch("interp_kernel");
 }
 

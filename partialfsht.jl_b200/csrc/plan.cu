@@ -916,21 +916,19 @@ int64_t plan_bytes(const pfsht_plan* p) {
     return bytes;
 }
 
-int plan_forward_after_ring(pfsht_plan* p, double2* f, cudaStream_t s, bool in_batch) {
+int plan_forward_after_ring(pfsht_plan* p, double2* f, cudaStream_t s) {
     StageClock* clk = &p->clk;
-    NufftGrid g = p->ng;
-    g.in_batch = in_batch ? 1 : 0;
     if (p->kind == kDirect) {
         PF_TRY(direct_phase_sum(p->H.as<double2>(), p->phi_pts.as<double>(), p->M, p->L, p->B, f, s));
         clock_mark(clk, kStDirect, s);
         return 0;
     }
-    if (g.cols) return nufft_type2_cols(g, p->nd, p->H.as<double2>(), f, p->B, +1, s, clk);
+    if (p->ng.cols) return nufft_type2_cols(p->ng, p->nd, p->H.as<double2>(), f, p->B, +1, s, clk);
     PF_CUFFT(cufftSetStream(p->fth, s));
     PF_CUFFT(cufftExecZ2Z(p->fth, p->H.as<cufftDoubleComplex>(), p->H.as<cufftDoubleComplex>(),
                           CUFFT_FORWARD));
     clock_mark(clk, kStFftThetaFwd, s);
-    return nufft_type2(g, p->nd, p->H.as<double2>(), f, p->B, +1, s, clk);
+    return nufft_type2(p->ng, p->nd, p->H.as<double2>(), f, p->B, +1, s, clk);
 }
 
 int plan_adjoint_before_ring(pfsht_plan* p, const double2* f, cudaStream_t s) {

@@ -125,7 +125,7 @@ struct DeviceGuard {
 
 // The pieces of one apply around its ring pass: the forward after the ring pass (FFT along
 // Theta and NUFFT type 2, or the Direct leaf's phase sum) and the adjoint before it.
-int plan_forward_after_ring(pfsht_plan* p, double2* f, cudaStream_t s, bool in_batch = false);
+int plan_forward_after_ring(pfsht_plan* p, double2* f, cudaStream_t s);
 int plan_adjoint_before_ring(pfsht_plan* p, const double2* f, cudaStream_t s);
 
 // The host-buffer apply without its final synchronisation: copies in (the coefficient
