@@ -1670,9 +1670,9 @@ int build_ring_merged(const std::vector<RingBatchPlan>& plans, bool adjoint, Rin
     // Heaviest first, so that the last items to end are short ones, but only by classes of a factor of four,
     // and plan by plan within a class: neighbouring warps then read the same plan's columns and
     // coefficients. Strictly by cost the plans alternate, the more so the more items have nearly the same
-    // cost: 64 plans (adjoint / forward) 6.57 / 3.84 ms, in classes of 1.2 6.19 / 3.65, of 2 6.02 / 3.59, of 4
-    // 5.96 / 3.57, plan by plan alone 5.93 / 3.60; 16 plans with a few large ones 1.57 / 1.18, 1.57 / 1.18,
-    // 1.55 / 1.18, 1.51 / 1.18, 1.51 / 1.24
+    // cost: 64 plans (adjoint / forward) 6.55 / 3.93 ms, in classes of 1.2 6.18 / 3.76, of 2 6.01 / 3.70, of 4
+    // 5.95 / 3.69, plan by plan alone 5.89 / 3.70; 16 plans with a few large ones 1.58 / 1.18, 1.57 / 1.17,
+    // 1.51 / 1.17, 1.51 / 1.18, 1.49 / 1.25
     auto cost_class = [](int64_t cost) {
         int k = 0;
         for (; cost >= 4; cost /= 4) ++k;
