@@ -708,7 +708,10 @@ ring_fwd_split_kernel(RingTables t, RingOut o, const RingItem* __restrict__ bloc
 // e^{+-i m phi} to the points' sums in registers, so no column array is written and read back
 // (49,152 points at lmax 191: 300 MB each way, and 125 us in a kernel of one thread per point that
 // summed the orders one after the other, and took 44 us for 400 points at lmax 64).
-// The groups' sums are added in a fixed order by direct_parts_kernel.
+// The groups' sums are added in a fixed order by direct_parts_kernel. FP64 issue bounds it (66 percent of
+// the pipe). Blocks per SM: with one less (nothing spills) lmax 191 takes 527 / 892 / 1598 us with one, two
+// and four transforms instead of 537 / 920 / 1598, and 400 points at lmax 64 19.3 / 20.1 / 22.2 instead of
+// 19.5 / 20.3 / 27.1.
 // ---------------------------------------------------------------------------------------
 constexpr int kDirectWarps = 4;
 template <int R, int NB>
